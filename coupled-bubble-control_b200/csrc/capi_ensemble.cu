@@ -167,6 +167,11 @@ static G grid_sizes(cbc_context* ctx, const cbc_spec* spec, const cbc_work* w) {
     g.threads[b] = block_threads_for(w->bucket_K[b], spec->nk, spec->lin_solver, max_block_smem(ctx->device),
                                      kExclusiveThreads);
     g.smem[b] = max_block_smem(ctx->device);
+    if (duo_form(w->bucket_K[b], spec->lin_solver)) {
+      // two-lane form: DUO_BLOCKS blocks of two warps fill the SM between them
+      g.first[b] = n * DUO_BLOCKS;
+      g.smem[b] = (g.smem[b] / DUO_BLOCKS - 1024) & ~(size_t)15;
+    }
     excl_sms += n;
   }
   const float rest = 1.f - (float)excl_sms / (float)ctx->sm_count;
@@ -183,9 +188,8 @@ static G grid_sizes(cbc_context* ctx, const cbc_spec* spec, const cbc_work* w) {
     if (w->blocks_per_sm && w->blocks_per_sm[b] > 0 && w->blocks_per_sm[b] < per_sm)
       full = (int)((float)(w->blocks_per_sm[b] * ctx->sm_count) * rest);
     if (full < 1) full = 1;
-    const int per_warp = (32 / K < g.slots[b]) ? 32 / K : g.slots[b];
-    const long long warps_needed = ((long long)(end - begin) + per_warp - 1) / per_warp;
-    const long long blocks_needed = (warps_needed * 32 + threads - 1) / threads;
+    const int per_block = systems_per_block(K, spec->lin_solver, threads, g.slots[b]);
+    const long long blocks_needed = ((long long)(end - begin) + per_block - 1) / per_block;
     if (full > blocks_needed) full = (int)blocks_needed;
     if (w->share) {
       float sh = w->share[b];

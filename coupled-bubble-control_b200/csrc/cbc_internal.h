@@ -14,6 +14,7 @@
 
 #include <type_traits>
 #include "ckm1d_core.cuh"
+#include "duo_core.cuh"
 
 #define CBC_MAX_BUCKETS 32   // two launches per bucket fit CBC_SIDE_STREAMS
 #define CBC_SIDE_STREAMS 64
@@ -129,16 +130,34 @@ constexpr size_t kScheduleBytes = kHeadBytes + 2 * sizeof(long long);
 // once per device.  *out stays NULL for device ordinals beyond its table.
 cudaError_t noalloc_scratch_address(int device, void** out);
 
+// Systems of this many bubbles and this solver run on the two-lane form
+// (duo_core.cuh): one system per block of DUO_THREADS threads.
+inline bool duo_form(int K, int lin) { return K > 16 && lin == LIN_RICHARDSON; }
+
+// Dynamic shared memory of a block of `threads` threads.
+inline size_t kernel_smem(int K, int nk, int lin, int threads) {
+  if (duo_form(K, lin)) return sizeof(double) * (size_t)duo_smem_doubles(nk);
+  const int warp = smem_doubles_per_warp(K, nk, lin);
+  return sizeof(double) * (size_t)warp * (threads / 32);
+}
+
 // Threads per block for a kernel of K bubbles per system: `requested`, cut
-// to whole warps whose shared memory fits the device's per-block limit
-// (K = 32 with its partner coefficients or augmented rows in shared memory
-// needs ~67 KB per warp, so at most three warps per block).
+// to whole warps whose shared memory fits the device's per-block limit (the
+// direct solve at K = 32 keeps its augmented rows there: ~64 KB per warp).
 inline int block_threads_for(int K, int nk, int lin, size_t max_block_smem, int requested) {
-  const size_t per_warp = sizeof(double) * (size_t)smem_doubles_per_warp(K, nk, lin);
+  if (duo_form(K, lin)) return DUO_THREADS;
+  const size_t per_warp = kernel_smem(K, nk, lin, 32);
   int warps = requested / 32;
   if (per_warp > 0 && (size_t)warps * per_warp > max_block_smem) warps = (int)(max_block_smem / per_warp);
   if (warps < 1) warps = 1;
   return warps * 32;
+}
+
+// Systems a block holds at once; slots: at most this many per warp.
+inline int systems_per_block(int K, int lin, int threads, int slots) {
+  if (duo_form(K, lin)) return 1;
+  const int fit = 32 / K;
+  return (fit < slots ? fit : slots) * (threads / 32);
 }
 
 // Smallest power-of-two instantiation that holds K bubbles per system.

@@ -42,9 +42,12 @@
 // rematerialising every 64-bit immediate in registers; the host (and the CPU
 // oracle) reads the identical constexpr values.
 #if defined(__CUDACC__)
+#ifndef CBCM_TABLE_CONST
+#define CBCM_TABLE_CONST const  // empty: the compiler may not fold the values into immediates
+#endif
 #define CBCM_TABLE(name, ...)                                  \
   static constexpr double name##_h[] = {__VA_ARGS__};          \
-  static __constant__ const double name##_d[] = {__VA_ARGS__};
+  static __constant__ CBCM_TABLE_CONST double name##_d[] = {__VA_ARGS__};
 #else
 #define CBCM_TABLE(name, ...) static constexpr double name##_h[] = {__VA_ARGS__};
 #endif

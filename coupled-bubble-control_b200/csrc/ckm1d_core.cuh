@@ -5,10 +5,9 @@
 // Everything that couples bubbles (coupling terms, the implicit-coupling
 // iteration, reductions for norms, error ratio and the collision event) is
 // exchanged inside the warp -- full-warp __shfl_sync, or per-warp
-// shared-memory records ordered by __syncwarp (partner states; the iterates
-// for K > 8) -- so no block barrier and no shared-memory atomics are needed
-// (the reference synchronises the
-// whole block 4x per Richardson iteration, ckm1d_def.py:303-404).  Control flow
+// shared-memory records ordered by __syncwarp (partner states) -- so no block
+// barrier and no shared-memory atomics are needed (the reference synchronises
+// the whole block 4x per Richardson iteration, ckm1d_def.py:303-404).  Control flow
 // that contains shuffles is warp-uniform; per-system decisions only select
 // values.  Per-system scalars (t, h, event value, ...) are held redundantly by
 // every lane of the group and stay identical because every lane computes them
@@ -32,6 +31,9 @@
 // Per-warp shared memory (WarpSmem): the group's harmonic constants, the
 // lane's 13 bubble constants (+2 derived) and the six stage derivatives.
 // Keeping these out of registers lets more warps stay resident.
+//
+// This file holds the Richardson form for 1 to 16 bubbles and the direct solve
+// for any number; Richardson above 16: two lanes per bubble (duo_core.cuh).
 #pragma once
 
 #include <stdint.h>
@@ -254,14 +256,14 @@ __device__ __forceinline__ void store_bubble_consts(const WarpSmem& w, const Geo
 
 __device__ __forceinline__ double upv(const WarpSmem& w, const Geo& g, int p) { return w.up[p * 32 + g.lane]; }
 
-// Per-system harmonic constants, component-major: hc[(7k + c) * G + grp].
+// Per-system harmonic constants, component-major: hc[(7k + c) * stride] (in a
+// warp's table stride G, first element grp).
 //   c = 0 w0*omega, 1 phase, 2 l0*wave, 3 PA, 4 PA*omega, 5 PA*wave, 6 PA*u0
 // Written by lane 0 of the group from system parameters sp1 = 1/omega_ref,
 // sp2 = lambda_ref/2pi, sp4 = 1/(rho c) and the control parameters
 // cp[m * cp_stride], m = 0..4nk-1 (PA, omega, phase, wave number).
-__device__ __forceinline__ void store_harmonics(const WarpSmem& w, const Geo& g, double sp1, double sp2,
-                                                double sp4, const double* cp, int nk,
-                                                long long cp_stride) {
+__device__ __forceinline__ void store_harmonics(double* hc, int stride, double sp1, double sp2, double sp4,
+                                                const double* cp, int nk, long long cp_stride) {
   // acoustic_field_1d (ckm1d_def.py:95-97): w0 = 2pi sp[1], l0 = 2pi sp[2], u0 = sp[4]
   const double w0 = TWO_PI * sp1;
   const double l0 = TWO_PI * sp2;
@@ -269,14 +271,14 @@ __device__ __forceinline__ void store_harmonics(const WarpSmem& w, const Geo& g,
   for (int k = 0; k < nk; ++k) {
     const double amps = cp[k * cp_stride], omega = cp[(nk + k) * cp_stride],
                  phase = cp[(2 * nk + k) * cp_stride], wave = cp[(3 * nk + k) * cp_stride];
-    double* h = w.hc + (HC_PER_K * k) * g.G + g.grp;
-    h[0 * g.G] = w0 * omega;
-    h[1 * g.G] = phase;
-    h[2 * g.G] = l0 * wave;
-    h[3 * g.G] = amps;
-    h[4 * g.G] = amps * omega;
-    h[5 * g.G] = amps * wave;
-    h[6 * g.G] = amps * u0;
+    double* h = hc + (HC_PER_K * k) * stride;
+    h[0 * stride] = w0 * omega;
+    h[1 * stride] = phase;
+    h[2 * stride] = l0 * wave;
+    h[3 * stride] = amps;
+    h[4 * stride] = amps * omega;
+    h[5 * stride] = amps * wave;
+    h[6 * stride] = amps * u0;
   }
 }
 
@@ -612,7 +614,7 @@ __device__ __forceinline__ void lu_solve_smem(const Geo& g, const WarpSmem& W, d
 // fixed the harmonic loops have no branches, so the independent sin/cos,
 // log/exp and division chains of the bubble interleave.
 template <int KB, int KC, int LIN, int NKC, int ACC>
-__device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const WarpSmem& W, const MView& M,
+__device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const WarpSmem& W,
                                          double sp0, double sp3, bool on, double t, const double y[4],
                                          double dy[4], bool& conv, int& iters) {
   const int nk = NKC > 0 ? NKC : P.nk;
@@ -893,15 +895,15 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
 // forms of the benchmarked workloads; any other form uses the general one.
 // P is uniform over a launch, so the branch never diverges.
 template <int KB, int KC, int LIN>
-__device__ __forceinline__ void rhs(const Geo& g, const Params& P, const WarpSmem& W, const MView& M,
+__device__ __forceinline__ void rhs(const Geo& g, const Params& P, const WarpSmem& W,
                                     double sp0, double sp3, bool on, double t, const double y[4],
                                     double dy[4], bool& conv, int& iters) {
   if (P.nk == 2 && P.ac == 2)
-    rhs_form<KB, KC, LIN, 2, 2>(g, P, W, M, sp0, sp3, on, t, y, dy, conv, iters);
+    rhs_form<KB, KC, LIN, 2, 2>(g, P, W, sp0, sp3, on, t, y, dy, conv, iters);
   else if (P.nk == 2 && P.ac == 1)
-    rhs_form<KB, KC, LIN, 2, 1>(g, P, W, M, sp0, sp3, on, t, y, dy, conv, iters);
+    rhs_form<KB, KC, LIN, 2, 1>(g, P, W, sp0, sp3, on, t, y, dy, conv, iters);
   else
-    rhs_form<KB, KC, LIN, 0, -1>(g, P, W, M, sp0, sp3, on, t, y, dy, conv, iters);
+    rhs_form<KB, KC, LIN, 0, -1>(g, P, W, sp0, sp3, on, t, y, dy, conv, iters);
 }
 
 // Exact sample time k of the grid dense mode.
@@ -935,6 +937,21 @@ __device__ __forceinline__ void prologue(LaneState& S, const Params& P, double g
   S.lin_iters = 0;
 }
 
+// Whether a system just loaded stores a dense sample before its first step.
+__device__ __forceinline__ bool first_sample(const LaneState& S, const Params& P) {
+  if (!S.active || S.idx >= P.ndo) return false;
+  return P.dense_mode == 0 ? S.dnext <= S.t : S.t >= grid_time(S, S.idx, P.ndo);
+}
+
+// Advances the dense schedule after that sample.
+__device__ __forceinline__ void first_stored(LaneState& S, const Params& P) {
+  S.idx += 1;
+  if (P.dense_mode == 0) {
+    const double nx = S.t + S.ddt;
+    S.dnext = nx < S.t_end ? nx : S.t_end;
+  }
+}
+
 // State at Cash-Karp stage ST: y + h * sum_{m < ST} b[ST][m] k_m, the sum
 // accumulated in increasing m (coefficients and loop fully compile-time).
 template <int ST>
@@ -952,8 +969,7 @@ __device__ __forceinline__ void stage_state(const double* ks, double h, const do
 // (stepper.py:362-677).  Returns true (per lane) if a dense sample must be
 // stored after this step; the caller writes it.
 template <int KB, int KC, int LIN>
-__device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSmem& W, const MView& M,
-                                     LaneState& S) {
+__device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSmem& W, LaneState& S) {
   const bool on = S.active;
   double h = S.h;
   if (h < P.min_step) h = P.min_step;
@@ -993,7 +1009,7 @@ __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSm
     double kk[4];
     bool cv;
     int it;
-    rhs<KB, KC, LIN>(g, P, W, M, S.sp0, S.sp3, on, ts, ys, kk, cv, it);
+    rhs<KB, KC, LIN>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, cv, it);
 #pragma unroll
     for (int c = 0; c < 4; ++c) ks[(st * 4 + c) * 32] = kk[c];
     if (on) {

@@ -60,6 +60,16 @@ cudaError_t launch_ensemble_bucket(const EnsLayout& E, const Params& P, const in
                                    cudaStream_t stream, size_t smem_bytes = 0, int slots = 32, int mb = 0);
 // Writes the device clock (%globaltimer, ns) to *epoch.
 cudaError_t launch_stamp(long long* epoch, cudaStream_t stream);
+// The same for one instantiation (KB, KC) of the kernels (see dispatch_k), and
+// its resident blocks per SM: defined in ensemble_kernel.cuh, instantiated by
+// kernels_k.cu.
+template <int KB, int KC>
+cudaError_t launch_ensemble_k(const EnsLayout& E, const Params& P, const int* order, int begin, int end, int K,
+                              int* head, long long max_steps, int steps_total, const long long* epoch,
+                              long long budget_ns, int blocks, int threads, cudaStream_t stream, size_t smem_bytes,
+                              int slots, int mb);
+template <int KB, int KC>
+cudaError_t occupancy_k(int K, int nk, int threads, int lin, int mb, int* n);
 size_t max_block_smem(int device);
 int resident_blocks(int K, int nk, int threads, int lin = LIN_RICHARDSON, int mb = 0);
 

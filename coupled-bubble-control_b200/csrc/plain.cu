@@ -1,166 +1,18 @@
-// plain.cu -- reference-layout CKM1D integrator (the drop-in solver) and the
-// context entry points of libcbc_b200.so.
-//
-// plain_kernel<KB> is the one-launch-per-K form: a static mapping of systems to
-// warps (floor(32/K) systems per warp, one lane per bubble) over the caller's
-// reference-layout buffers, advancing each system by at most `budget` steps.
-// It replaces the fused kernel of the reference
-// (backends/numba/rkck45_coupled_numba_stepper.py:116-706) and cbc_solve
-// replaces the host launch loop (backends/numba/rkck45_coupled_numba_solver.py:29-91).
+// plain.cu -- the reference-layout solve and the context entry points of
+// libcbc_b200.so.  cbc_solve replaces the host launch loop of the reference
+// (backends/numba/rkck45_coupled_numba_solver.py:29-91); its kernels are in
+// plain_kernel.cuh.
+#include <new>
+
 #include "cbc_internal.h"
+#include "plain.h"
 
 namespace cbc {
-
-struct RefLayout {
-  int ns, ups, tile;
-  double* actual_time;
-  const double* time_end;
-  const double* time_begin;
-  double* time_step;
-  double* actual_state;
-  const double* unit_params;
-  const double* system_params;
-  const double* control_params;
-  const double* coupling;
-  int* dense_index;
-  double* dense_time;
-  double* dense_state;
-  double* actual_event;
-  int* status;
-  int* total_steps;
-  int* rejected_steps;
-  int* conv_success;
-  int* conv_failures;
-  long long* lin_iters;
-};
-
-template <int KB>
-__device__ __forceinline__ void ref_store_dense(const RefLayout& L, const LaneState& S, const Geo& g,
-                                                long long s, int slot) {
-  const long long NST = (long long)L.ns * L.tile;
-  if (g.li == 0) L.dense_time[(long long)slot * L.ns + s] = S.t;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) L.dense_state[((long long)slot * 4 + c) * NST + s * L.tile + g.li] = S.y[c];
-}
-
-template <int KB, int KC, int LIN>
-__global__ void __launch_bounds__(128, min_blocks_for(KB)) plain_kernel(RefLayout L, Params P, long long budget, int final_launch,
-                                                    int* active_counter) {
-  extern __shared__ __align__(16) double smem[];
-  const Geo g = make_geo(KC > 0 ? KC : L.ups);
-  const WarpSmem W = warp_smem(smem, L.ups, P.nk, LIN);
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long s = warp * g.G + g.grp;
-  const bool have = g.valid && s < L.ns;
-  const long long NST = (long long)L.ns * L.tile;
-  const long long lane_off = s * L.tile + g.li;
-
-  LaneState S;
-  MView M;
-  M.m = L.coupling + (have ? lane_off : 0);
-  M.sc = (long long)L.ups * NST;
-  M.sj = NST;
-  S.active = false;
-  S.status = ST_ACTIVE;
-  double g_store = 0.0;
-  if (have) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) S.y[c] = L.actual_state[c * NST + lane_off];
-    store_bubble_consts(W, g, L.unit_params + lane_off, NST);
-    store_coupling(W, g, M);
-    S.sp0 = L.system_params[0 * (long long)L.ns + s];
-    S.sp3 = L.system_params[3 * (long long)L.ns + s];
-    S.t = L.actual_time[s];
-    S.t_end = L.time_end[s];
-    S.t_begin = L.time_begin[s];
-    S.h = L.time_step[s];
-    S.idx = (P.ndo > 0) ? L.dense_index[s] : 0;
-    g_store = L.actual_event[s];
-    const double prev = (P.ndo > 0 && S.idx > 0) ? L.dense_time[(long long)(S.idx - 1) * L.ns + s] : 0.0;
-    prologue(S, P, g_store, prev, L.status[s]);
-    if (g.li == 0)
-      store_harmonics(W, g, L.system_params[1 * (long long)L.ns + s], L.system_params[2 * (long long)L.ns + s],
-                      L.system_params[4 * (long long)L.ns + s], L.control_params + s, P.nk, L.ns);
-  }
-  __syncwarp();
-
-  // first dense sample and initial event value (stepper.py:333-358)
-  if (S.active && P.ndo > 0) {
-    bool st = false;
-    if (P.dense_mode == 0) st = (S.idx < P.ndo) && (S.dnext <= S.t);
-    else st = (S.idx < P.ndo) && (S.t >= grid_time(S, S.idx, P.ndo));
-    if (st) {
-      ref_store_dense<KB>(L, S, g, s, S.idx);
-      S.idx += 1;
-      if (P.dense_mode == 0) {
-        const double nx = S.t + S.ddt;
-        S.dnext = nx < S.t_end ? nx : S.t_end;
-      }
-    }
-  }
-  {
-    const double g0 = group_event<KB>(S.y, upv(W, g, 12), g, P.col);
-    if (S.active) S.g_old = g0;
-  }
-
-  for (long long it = 0; it < budget; ++it) {
-    if (!__any_sync(FULL, S.active)) break;
-    const bool st = step<KB, KC, LIN>(g, P, W, M, S);
-    if (st) ref_store_dense<KB>(L, S, g, s, S.idx);
-    after_store(S, P, st);
-  }
-
-  if (have) {
-    if (S.status == ST_ACTIVE && final_launch) S.status = ST_MAX_STEPS;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) L.actual_state[c * NST + lane_off] = S.y[c];
-    if (g.li == 0) {
-      L.actual_time[s] = S.t;
-      L.time_step[s] = S.h;
-      L.actual_event[s] = S.g_old;
-      L.status[s] = S.status;
-      if (P.ndo > 0) L.dense_index[s] = S.idx;
-      if (L.total_steps) L.total_steps[s] += S.steps;
-      if (L.rejected_steps) L.rejected_steps[s] += S.rejected;
-      if (L.conv_success) L.conv_success[s] += S.conv_ok;
-      if (L.conv_failures) L.conv_failures[s] += S.conv_fail;
-      if (L.lin_iters) L.lin_iters[s] += S.lin_iters;
-      if (S.status == ST_ACTIVE && active_counter) atomicAdd(active_counter, 1);
-    }
-  }
-}
-
-template <int KB, int KC, int LIN>
-cudaError_t launch_plain(const RefLayout& L, const Params& P, long long budget, int final_launch, int* counter,
-                         cudaStream_t stream) {
-  const int G = 32 / L.ups;
-  const long long warps = (L.ns + G - 1) / G;
-  int dev = 0;
-  cudaError_t de = cudaGetDevice(&dev);
-  if (de != cudaSuccess) return de;
-  int cap = 0;
-  de = cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (de != cudaSuccess) return de;
-  const int threads = block_threads_for(L.ups, P.nk, LIN, (size_t)cap, 128);
-  const long long blocks = (warps * 32 + threads - 1) / threads;
-  const size_t shmem = sizeof(double) * (size_t)smem_doubles_per_warp(L.ups, P.nk, LIN) * (threads / 32);
-  if (shmem > 48 * 1024) {
-    cudaError_t e =
-        cudaFuncSetAttribute(plain_kernel<KB, KC, LIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
-    if (e != cudaSuccess) return e;
-  }
-  plain_kernel<KB, KC, LIN><<<(unsigned)blocks, threads, shmem, stream>>>(L, P, budget, final_launch, counter);
-  return cudaGetLastError();
-}
 
 cudaError_t launch_plain_any(const RefLayout& L, const Params& P, long long budget, int final_launch,
                              int* counter, cudaStream_t stream) {
   return dispatch_k(L.ups, [&](auto kb, auto kc) {
-    return dispatch_lin(P.lin, [&](auto lin) {
-      return launch_plain<decltype(kb)::value, decltype(kc)::value, decltype(lin)::value>(L, P, budget,
-                                                                                         final_launch, counter,
-                                                                                         stream);
-    });
+    return launch_plain_k<decltype(kb)::value, decltype(kc)::value>(L, P, budget, final_launch, counter, stream);
   });
 }
 
