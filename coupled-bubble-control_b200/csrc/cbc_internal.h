@@ -15,6 +15,7 @@
 #include <type_traits>
 #include "ckm1d_core.cuh"
 #include "duo_core.cuh"
+#include "wide_core.cuh"
 
 #define CBC_MAX_BUCKETS 32   // two launches per bucket fit CBC_SIDE_STREAMS
 #define CBC_SIDE_STREAMS 64
@@ -134,10 +135,13 @@ cudaError_t noalloc_scratch_address(int device, void** out);
 // (duo_core.cuh): one system per block of DUO_THREADS threads.
 inline bool duo_form(int K, int lin) { return K > 16 && lin == LIN_RICHARDSON; }
 
+// Of these on the form for 9 to 16 bubbles (wide_core.cuh).
+inline bool wide_form(int K, int lin) { return K > 8 && K <= 16 && lin == LIN_RICHARDSON; }
+
 // Dynamic shared memory of a block of `threads` threads.
 inline size_t kernel_smem(int K, int nk, int lin, int threads) {
   if (duo_form(K, lin)) return sizeof(double) * (size_t)duo_smem_doubles(nk);
-  const int warp = smem_doubles_per_warp(K, nk, lin);
+  const int warp = wide_form(K, lin) ? wide_smem_doubles(K, nk) : smem_doubles_per_warp(K, nk, lin);
   return sizeof(double) * (size_t)warp * (threads / 32);
 }
 

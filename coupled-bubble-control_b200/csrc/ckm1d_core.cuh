@@ -32,8 +32,10 @@
 // lane's 13 bubble constants (+2 derived) and the six stage derivatives.
 // Keeping these out of registers lets more warps stay resident.
 //
-// This file holds the Richardson form for 1 to 16 bubbles and the direct solve
-// for any number; Richardson above 16: two lanes per bubble (duo_core.cuh).
+// This file holds the Richardson form for 1 to 8 bubbles and the direct solve
+// for any number.  Other Richardson forms: 9 to 16 bubbles with
+// the coefficients in registers (wide_core.cuh), two lanes per bubble above
+// (duo_core.cuh).
 #pragma once
 
 #include <stdint.h>
@@ -176,17 +178,13 @@ enum : int { LIN_RICHARDSON = 0, LIN_LU = 1 };
 // region (and every warp's carve-up) stays 16-byte aligned for double2 access.
 __host__ __device__ inline int hc_doubles(int K, int nk) { return (HC_PER_K * nk * (32 / K) + 1) & ~1; }
 
-// Matrix region per warp:
-//   Richardson, K <= 8: none (the partner coefficients live in registers);
-//   Richardson, K > 8:  the partner coefficients as double2 records
-//                       [K-1][(A,B), (C,D)][32] (kept out of registers: local
-//                       memory would spill to L2);
-//   direct, K <= 8:     staging of the four coefficient blocks by absolute
-//                       column, [4][K][32], read back into register rows;
-//   direct, K > 8:      the two augmented rows of every lane, [2][2K+1][32].
+// Matrix region per warp (direct solve only):
+//   K <= 8: staging of the four coefficient blocks by absolute column,
+//           [4][K][32], read back into register rows;
+//   K > 8:  the two augmented rows of every lane, [2][2K+1][32].
 __host__ __device__ inline int mat_doubles(int K, int lin) {
-  if (K <= 8) return lin == LIN_LU ? 4 * K * 32 : 0;
-  return lin == LIN_LU ? 2 * (2 * K + 1) * 32 : 4 * (K - 1) * 32;
+  if (lin != LIN_LU) return 0;
+  return K <= 8 ? 4 * K * 32 : 2 * (2 * K + 1) * 32;
 }
 __host__ __device__ inline int pv_doubles(int K, int lin) {
   return (K > 8 && lin == LIN_LU) ? (((32 / K) * (2 * K + 1) + 1) & ~1) : 0;
@@ -357,8 +355,8 @@ __device__ __forceinline__ double group_sum_full(double v) {
 // Residual r = b - A v of the implicit coupling system for this lane's bubble,
 // A = I + off-diagonal partner blocks.  Partner distance d = 1..K-1 goes to
 // accumulation chain (d - 1) mod 4 (increasing d within a chain); the chains
-// are then combined by the open pairwise tree.  Coefficients from registers
-// (K <= 8) or from the lane's shared-memory columns (K > 8).
+// accumulation chain (d - 1) mod 4 (increasing d within a chain); the chains
+// are then combined by the open pairwise tree.
 template <int KB>
 __device__ __forceinline__ void residual(const Geo& g, const double* Am, const double* Bm, const double* Cm,
                                          const double* Dm, double cpf0, double b0, double b1, double vr,
@@ -372,37 +370,6 @@ __device__ __forceinline__ void residual(const Geo& g, const double* Am, const d
       const int c = (d - 1) & 3;
       ar[c] = fma(Am[d], vrj, fma(Bm[d], vtj, ar[c]));
       at[c] = fma(Cm[d], vrj, fma(Dm[d], vtj, at[c]));
-    }
-  const int nc = g.K - 1 < 4 ? g.K - 1 : 4;
-  const double sr = tree_open(ar, nc);
-  const double st = tree_open(at, nc);
-  r0 = b0 - fma(sr, cpf0, vr);
-  r1 = b1 - (st + vt);
-}
-
-// The same for K > 8, from shared memory: the coefficients of partner
-// distance d as two double2 records per lane, (A, B) at [(d - 1) 2][lane] and
-// (C, D) at [(d - 1) 2 + 1][lane]; the partner iterates through the warp's
-// exchange records (one 16-byte store per lane and one 16-byte load per
-// partner, instead of two 64-bit shuffles per partner).  Same values and the
-// same accumulation order as the register form.
-template <int KB>
-__device__ __forceinline__ void residual_smem(const Geo& g, const WarpSmem& W, double cpf0, double b0, double b1,
-                                              double vr, double vt, double& r0, double& r1) {
-  double ar[4] = {0.0, 0.0, 0.0, 0.0}, at[4] = {0.0, 0.0, 0.0, 0.0};
-  const double2* m2 = reinterpret_cast<const double2*>(W.mat) + g.lane;
-  double2* xr = reinterpret_cast<double2*>(W.xv);
-  __syncwarp();
-  xr[g.lane] = make_double2(vr, vt);
-  __syncwarp();
-#pragma unroll
-  for (int d = 1; d < KB; ++d)
-    if (d < g.K) {
-      const double2 vj = xr[partner_rec(g, d)];
-      const int c = (d - 1) & 3;
-      const double2 ab = m2[(2 * (d - 1)) * 32], cd = m2[(2 * (d - 1) + 1) * 32];
-      ar[c] = fma(ab.x, vj.x, fma(ab.y, vj.y, ar[c]));
-      at[c] = fma(cd.x, vj.x, fma(cd.y, vj.y, at[c]));
     }
   const int nc = g.K - 1 < 4 ? g.K - 1 : 4;
   const double sr = tree_open(ar, nc);
@@ -673,10 +640,10 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
 
   // ---- explicit coupling + matrix of the implicit system over partners ----
   // The partner coefficients A, B, C, D of the implicit system go to
-  // registers (Richardson, K <= 8), to the lane's shared-memory columns by
-  // partner distance (Richardson, K > 8) or by absolute partner column (the
-  // direct solve: its staging area for K <= 8, its augmented rows for K > 8).
-  constexpr bool REG = (KB <= 8) && (LIN == LIN_RICHARDSON);
+  // registers (Richardson) or to the lane's shared-memory columns by absolute
+  // partner column (the direct solve: its staging area for K <= 8, its
+  // augmented rows for K > 8).
+  constexpr bool REG = LIN == LIN_RICHARDSON;
   double g0 = 0.0, g1 = 0.0, tn = 0.0, tg2 = 0.0, tg3 = 0.0;
   double Am[REG ? KB : 1], Bm[REG ? KB : 1], Cm[REG ? KB : 1], Dm[REG ? KB : 1];
   double* mcol = W.mat + g.lane;
@@ -739,10 +706,6 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
           Bm[d] = b_;
           Cm[d] = c_;
           Dm[d] = d_;
-        } else if constexpr (LIN == LIN_RICHARDSON) {
-          double2* mcol2 = reinterpret_cast<double2*>(W.mat) + g.lane;
-          mcol2[(2 * (d - 1)) * 32] = make_double2(a_, b_);
-          mcol2[(2 * (d - 1) + 1) * 32] = make_double2(c_, d_);
         } else {
           const int j = partner_lane(g, d) - g.base;   // absolute partner column
           if constexpr (KB <= 8) {
@@ -839,20 +802,17 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
   const bool full_groups = (g.K == KB);
   const int maxit = P.lin_max_iter;
   double r0, r1;
-  if constexpr (REG) residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, vr, vt, r0, r1);
-  else residual_smem<KB>(g, W, cpf0, b0, b1, vr, vt, r0, r1);
+  residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, vr, vt, r0, r1);
   for (int it = 0; it < maxit; it += 2) {
     if (__all_sync(FULL, found)) break;
     // iterate it: (vr, vt) with residual (r0, r1); iterate it + 1: (br, bt)
     const double br = fma(P.omega, r0, vr), bt = fma(P.omega, r1, vt);
     double q0, q1;
-    if constexpr (REG) residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, br, bt, q0, q1);
-    else residual_smem<KB>(g, W, cpf0, b0, b1, br, bt, q0, q1);
+    residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, br, bt, q0, q1);
     const bool two = it + 1 < maxit;   // the plain loop also tests iterate it + 1
     const double wr = fma(P.omega, q0, br), wt = fma(P.omega, q1, bt);
     double s0, s1;
-    if constexpr (REG) residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, wr, wt, s0, s1);
-    else residual_smem<KB>(g, W, cpf0, b0, b1, wr, wt, s0, s1);
+    residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, wr, wt, s0, s1);
     const double rra = fma(r0, r0, r1 * r1), rrb = fma(q0, q0, q1 * q1);
     double rna, rnb;
     if (full_groups) {

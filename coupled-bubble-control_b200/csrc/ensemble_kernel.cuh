@@ -20,6 +20,7 @@
 #include "cbc_internal.h"
 #include "ensemble.h"
 #include "duo_core.cuh"
+#include "wide_core.cuh"
 
 namespace cbc {
 
@@ -105,7 +106,7 @@ __device__ __forceinline__ void ens_write_scalars(const EnsLayout& E, const Para
                     S.c->conv_fail, S.c->lin_iters);
 }
 
-// ---- 1 to 16 bubbles, and the direct solve for any number (ckm1d_core.cuh) ----
+// ---- 1 to 8 bubbles, and the direct solve for any number (ckm1d_core.cuh) ----
 
 // Loads system s into this lane's slot (lane li of the group) and runs the
 // prologue.  Called only by lanes whose group claimed s.
@@ -244,6 +245,140 @@ __global__ void __launch_bounds__(128, min_blocks_variant(KB, MB))
   }
 }
 
+// 9 to 16 bubbles with the Richardson solve (wide_core.cuh):
+template <int KC>
+struct WideForm {
+  Geo g;
+  WideSmem W;
+  BubbleState S;
+
+  __device__ __forceinline__ WideForm(double* smem, int K, int nk, int slots)
+      : g(make_geo(KC > 0 ? KC : K, slots)), W(wide_smem(smem, g.K, nk)) {
+    S.c = W.cold + g.grp;
+    S.o = W.own + g.lane;
+    S.lead = g.valid && g.li == 0;
+    S.active = false;
+    S.status = ST_ACTIVE;
+  }
+  __device__ __forceinline__ void load(const EnsLayout& E, const Params& P, int s, int steps_total,
+                                       long long max_steps) {
+    const long long row = E.bubble_offset[s] + g.li;
+    ens_load_state(E, row, S.y);
+    ens_load_scalars(E, P, s, S);
+    wide_store_bubble(W, g, E.unit_params + row * E.up_stride, 1,
+                      MView{E.coupling + E.coupling_offset[s] + g.li, (long long)g.K * g.K, g.K});
+    const double* sp = E.system_params + (long long)s * E.sp_stride;
+    if (S.lead)
+      store_harmonics(W.hc + g.grp, g.G, sp[1], sp[2], sp[4], E.control_params + (long long)s * E.cp_stride, P.nk, 1);
+    ens_step_base(E, s, steps_total, max_steps, S);
+  }
+  __device__ __forceinline__ void begin(const EnsLayout& E, const Params& P, bool fresh, int s) {
+    if (fresh && first_sample(S, P)) {
+      ens_store_dense(E, S.t, S.y, S.c->boff, g.li, s, S.o->idx);
+      first_stored(S, P);
+    }
+    const double g0 = group_event<WIDE>(S.y, upv(W, g, 12), g, P.col);
+    if (fresh && S.active) S.g_old = g0;
+  }
+  __device__ __forceinline__ void write(const EnsLayout& E, const Params& P, int s) {
+    ens_write_state(E, S.c->boff + g.li, S.y);
+    if (S.lead) ens_write_scalars(E, P, s, S);
+  }
+  __device__ __forceinline__ void stop() {
+    S.status = ST_MAX_STEPS;
+    S.active = false;
+  }
+  __device__ __forceinline__ void advance(const EnsLayout& E, const Params& P, int s, long long max_steps) {
+    const bool stq = wide_step<KC>(g, P, W, S);
+    if (stq) ens_store_dense(E, S.t, S.y, S.c->boff, g.li, s, S.o->idx);
+    after_store(S, P, stq);
+    if (S.active && S.o->steps + S.c->step_base >= max_steps) stop();
+  }
+};
+
+// Persistent worker: warps claim systems of bucket [begin, end) of the work
+// list until it is empty.  All systems of a bucket have the same K.
+template <class Form>
+__device__ __forceinline__ void ensemble_worker(Form& f, const EnsLayout& E, const Params& P,
+                                                const int* __restrict__ order, int begin, int end, int* head,
+                                                long long max_steps, int steps_total, const long long* epoch,
+                                                long long budget_ns) {
+  const Geo& g = f.g;
+  const int lane = threadIdx.x & 31;
+  const bool leader = g.valid && g.li == 0;
+  int sys = -1;           // system in this lane's slot (-1: none)
+  bool drained = false;   // work list exhausted for this warp (warp-uniform)
+  const long long deadline = budget_ns > 0 ? epoch[0] + budget_ns : 0;
+  bool sliced_out = false;  // time slice over (warp-uniform); independent of drained
+
+  while (true) {
+    // ---- time slice over: stop every slot after its current step ----
+    if (deadline != 0 && !sliced_out) {
+      long long now = 0;
+      if (lane == 0) now = global_ns();
+      now = __shfl_sync(FULL, now, 0);
+      if (now >= deadline) {
+        sliced_out = true;
+        drained = true;
+      }
+    }
+    if (sliced_out && f.S.active) f.stop();
+    // ---- retire finished systems and refill empty slots (warp-uniform) ----
+    const bool retire = g.valid && sys >= 0 && !f.S.active;
+    if (__any_sync(FULL, retire)) {
+      if (retire) {
+        f.write(E, P, sys);
+        sys = -1;
+      }
+      __syncwarp();
+    }
+    const bool want = leader && sys < 0 && !drained;
+    const unsigned wmask = __ballot_sync(FULL, want);
+    if (wmask) {
+      int base_idx = 0;
+      if (lane == 0) base_idx = atomicAdd(head, __popc(wmask));
+      base_idx = __shfl_sync(FULL, base_idx, 0);
+      int claim = -1;
+      if (want) {
+        const int idx = begin + base_idx + __popc(wmask & ((1u << lane) - 1u));
+        claim = (idx < end) ? order[idx] : -1;
+      }
+      if (__any_sync(FULL, want && claim < 0)) drained = true;
+      // hand the claimed system id to every lane of the group
+      // (both shuffles are executed by every lane: never inside a
+      // short-circuit or a divergent branch)
+      const int got = __shfl_sync(FULL, claim, g.base);
+      const int leader_wanted = __shfl_sync(FULL, (int)want, g.base);
+      const bool fresh = g.valid && sys < 0 && got >= 0 && leader_wanted != 0;
+      if (fresh) {
+        sys = got;
+        if (leader && E.trace_load_ns) E.trace_load_ns[sys] = global_ns();
+        f.load(E, P, sys, steps_total, max_steps);
+      }
+      __syncwarp();
+      f.begin(E, P, fresh, sys);
+      // systems that arrive already finished go straight back out
+      continue;
+    }
+    if (!__any_sync(FULL, f.S.active)) {
+      if (!__any_sync(FULL, sys >= 0)) break;  // nothing left in any slot
+      continue;
+    }
+    // ---- one Cash-Karp step for every active slot ----
+    f.advance(E, P, sys, max_steps);
+  }
+}
+
+template <int KC>
+__global__ void __launch_bounds__(WIDE_THREADS, 1)
+    ensemble_wide_kernel(EnsLayout E, Params P, const int* __restrict__ order, int begin, int end, int K, int* head,
+                         long long max_steps, int steps_total, const long long* epoch, long long budget_ns,
+                         int slots) {
+  extern __shared__ __align__(16) double smem[];
+  WideForm<KC> f(smem, K, P.nk, slots);
+  ensemble_worker(f, E, P, order, begin, end, head, max_steps, steps_total, epoch, budget_ns);
+}
+
 // The same for 17 to 32 bubbles per system with the Richardson solve: one system
 // per block of two warps (duo_core.cuh).  KC: exact K, or 0 (read at run time).
 template <int KC>
@@ -355,6 +490,12 @@ cudaError_t launch_ensemble_k(const EnsLayout& E, const Params& P, const int* or
         if (e != cudaSuccess) return e;
         kernel<<<blocks, threads, shmem, stream>>>(E, P, order, begin, end, K, head, max_steps, steps_total, epoch,
                                                    budget_ns);
+      } else if constexpr (KB == 16 && LIN == LIN_RICHARDSON) {
+        const auto kernel = ensemble_wide_kernel<KC>;
+        const cudaError_t e = configure_kernel(kernel, shmem);
+        if (e != cudaSuccess) return e;
+        kernel<<<blocks, threads, shmem, stream>>>(E, P, order, begin, end, K, head, max_steps, steps_total, epoch,
+                                                   budget_ns, slots);
       } else {
         const auto kernel = ensemble_kernel<KB, KC, LIN, MB>;
         const cudaError_t e = configure_kernel(kernel, shmem);
@@ -375,6 +516,10 @@ cudaError_t occupancy_k(int K, int nk, int threads, int lin, int mb, int* n) {
       constexpr int LIN = decltype(li)::value, MB = KB <= 8 ? decltype(mbv)::value : 0;
       if constexpr (KB == 32 && LIN == LIN_RICHARDSON) {
         const auto kernel = ensemble_duo_kernel<KC>;
+        configure_kernel(kernel, shmem);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, threads, shmem);
+      } else if constexpr (KB == 16 && LIN == LIN_RICHARDSON) {
+        const auto kernel = ensemble_wide_kernel<KC>;
         configure_kernel(kernel, shmem);
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, threads, shmem);
       } else {

@@ -1,9 +1,11 @@
 // kernels_k.cu -- the batched and reference-layout kernels of one
 // instantiation: compiled once per (CBC_KB, CBC_KC) pair of dispatch_k, so that
 // the instantiations build in parallel.
-// Above 16 bubbles the matrix rows of a lane fill its registers, and tables that the
-// compiler may fold cost more of them (direct solve: 240 registers, 194 without).
-#if CBC_KB >= 32
+// Above 8 bubbles the matrix rows of a lane fill its registers, and tables that
+// the compiler may fold cost more of them (9 to 15 bubbles: 104 bytes spilled, 40
+// without; 16: 4, 0; direct solve: 254 registers, 194).  Up to 8 bubbles it is the
+// other way round (2 bubbles: 0 bytes folded, 24 without; direct solve 8, 242).
+#if CBC_KB >= 16
 #define CBCM_TABLE_CONST
 #endif
 #include "ensemble_kernel.cuh"

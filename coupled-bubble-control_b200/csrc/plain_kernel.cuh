@@ -9,6 +9,7 @@
 #include "cbc_internal.h"
 #include "duo_core.cuh"
 #include "plain.h"
+#include "wide_core.cuh"
 
 namespace cbc {
 
@@ -99,7 +100,7 @@ __device__ __forceinline__ void ref_write_scalars(const RefLayout& L, const Para
                     S.c->conv_fail, S.c->lin_iters, active_counter);
 }
 
-// One lane per bubble: 1 to 16 bubbles, and the direct solve (ckm1d_core.cuh).
+// One lane per bubble: 1 to 8 bubbles, and the direct solve (ckm1d_core.cuh).
 template <int KB, int KC, int LIN>
 __global__ void __launch_bounds__(128, min_blocks_for(KB))
     plain_kernel(RefLayout L, Params P, long long budget, int final_launch, int* active_counter) {
@@ -139,6 +140,54 @@ __global__ void __launch_bounds__(128, min_blocks_for(KB))
     after_store(S, P, st);
   }
 
+  if (have) {
+    if (S.status == ST_ACTIVE && final_launch) S.status = ST_MAX_STEPS;
+    ref_write_state(L, S.y, lane_off);
+    if (g.li == 0) ref_write_scalars(L, P, s, S, active_counter);
+  }
+}
+
+// The same for 9 to 16 bubbles with the Richardson solve (wide_core.cuh).
+template <int KC>
+__global__ void __launch_bounds__(WIDE_THREADS, 1)
+    plain_wide_kernel(RefLayout L, Params P, long long budget, int final_launch, int* active_counter) {
+  extern __shared__ __align__(16) double smem[];
+  const Geo g = make_geo(KC > 0 ? KC : L.ups);
+  const WideSmem W = wide_smem(smem, g.K, P.nk);
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long s = warp * g.G + g.grp;
+  const bool have = g.valid && s < L.ns;
+  const long long NST = (long long)L.ns * L.tile;
+  const long long lane_off = s * L.tile + g.li;
+
+  BubbleState S;
+  S.c = W.cold + g.grp;
+  S.o = W.own + g.lane;
+  S.lead = have && g.li == 0;
+  S.active = false;
+  S.status = ST_ACTIVE;
+  if (have) {
+    ref_load_state(L, lane_off, S.y);
+    ref_load(L, P, s, S);
+    wide_store_bubble(W, g, L.unit_params + lane_off, NST,
+                      MView{L.coupling + lane_off, (long long)L.ups * NST, NST});
+    if (g.li == 0) ref_store_harmonics(L, P, s, W.hc + g.grp, g.G);
+  }
+  __syncwarp();
+  if (have && first_sample(S, P)) {
+    ref_store_dense(L, S.t, S.y, g.li, s, S.o->idx);
+    first_stored(S, P);
+  }
+  {
+    const double g0 = group_event<WIDE>(S.y, upv(W, g, 12), g, P.col);
+    if (S.active) S.g_old = g0;
+  }
+  for (long long it = 0; it < budget; ++it) {
+    if (!__any_sync(FULL, S.active)) break;
+    const bool st = wide_step<KC>(g, P, W, S);
+    if (st) ref_store_dense(L, S.t, S.y, g.li, s, S.o->idx);
+    after_store(S, P, st);
+  }
   if (have) {
     if (S.status == ST_ACTIVE && final_launch) S.status = ST_MAX_STEPS;
     ref_write_state(L, S.y, lane_off);
@@ -211,7 +260,8 @@ cudaError_t launch_plain_k(const RefLayout& L, const Params& P, long long budget
       kernel<<<(unsigned)blocks, threads, shmem, stream>>>(L, P, budget, final_launch, counter);
       return cudaGetLastError();
     };
-    if constexpr (KB == 32 && LIN == LIN_RICHARDSON) return launch(plain_duo_kernel<KC>);
+    if constexpr (KB == 16 && LIN == LIN_RICHARDSON) return launch(plain_wide_kernel<KC>);
+    else if constexpr (KB == 32 && LIN == LIN_RICHARDSON) return launch(plain_duo_kernel<KC>);
     else return launch(plain_kernel<KB, KC, LIN>);
   });
 }
