@@ -15,6 +15,7 @@
 #include <type_traits>
 #include "ckm1d_core.cuh"
 #include "duo_core.cuh"
+#include "solo_core.cuh"
 #include "wide_core.cuh"
 
 #define CBC_MAX_BUCKETS 32   // two launches per bucket fit CBC_SIDE_STREAMS
@@ -135,13 +136,18 @@ cudaError_t noalloc_scratch_address(int device, void** out);
 // (duo_core.cuh): one system per block of DUO_THREADS threads.
 inline bool duo_form(int K, int lin) { return K > 16 && lin == LIN_RICHARDSON; }
 
-// Of these on the form for 9 to 16 bubbles (wide_core.cuh).
+// Of these on the one-lane form (solo_core.cuh): 32 systems per warp.
+inline bool solo_form(int K, int lin) { return K == 1 && lin == LIN_RICHARDSON; }
+
+// And of these on the form for 9 to 16 bubbles (wide_core.cuh).
 inline bool wide_form(int K, int lin) { return K > 8 && K <= 16 && lin == LIN_RICHARDSON; }
 
 // Dynamic shared memory of a block of `threads` threads.
 inline size_t kernel_smem(int K, int nk, int lin, int threads) {
   if (duo_form(K, lin)) return sizeof(double) * (size_t)duo_smem_doubles(nk);
-  const int warp = wide_form(K, lin) ? wide_smem_doubles(K, nk) : smem_doubles_per_warp(K, nk, lin);
+  const int warp = solo_form(K, lin)   ? solo_smem_doubles(nk)
+                   : wide_form(K, lin) ? wide_smem_doubles(K, nk)
+                                       : smem_doubles_per_warp(K, nk, lin);
   return sizeof(double) * (size_t)warp * (threads / 32);
 }
 
@@ -160,7 +166,7 @@ inline int block_threads_for(int K, int nk, int lin, size_t max_block_smem, int 
 // Systems a block holds at once; slots: at most this many per warp.
 inline int systems_per_block(int K, int lin, int threads, int slots) {
   if (duo_form(K, lin)) return 1;
-  const int fit = 32 / K;
+  const int fit = solo_form(K, lin) ? 32 : 32 / K;
   return (fit < slots ? fit : slots) * (threads / 32);
 }
 

@@ -32,10 +32,10 @@
 // lane's 13 bubble constants (+2 derived) and the six stage derivatives.
 // Keeping these out of registers lets more warps stay resident.
 //
-// This file holds the Richardson form for 1 to 8 bubbles and the direct solve
-// for any number.  Other Richardson forms: 9 to 16 bubbles with
-// the coefficients in registers (wide_core.cuh), two lanes per bubble above
-// (duo_core.cuh).
+// This file holds the Richardson form for 2 to 8 bubbles and the direct solve
+// for any number.  Other Richardson forms: one lane per system for a single
+// bubble (solo_core.cuh), one lane per bubble for 9 to 16 (wide_core.cuh), two
+// lanes per bubble above (duo_core.cuh).
 #pragma once
 
 #include <stdint.h>

@@ -1,5 +1,5 @@
 // cold_core.cuh -- what the Richardson forms outside ckm1d_core.cuh share
-// (wide_core.cuh, duo_core.cuh): a system's scalars in shared
+// (solo_core.cuh, wide_core.cuh, duo_core.cuh): a system's scalars in shared
 // memory, the right-hand side's parts as functions, the controller.
 //
 // Same operations in the same order as ckm1d_core.cuh.

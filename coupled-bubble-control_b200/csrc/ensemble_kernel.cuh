@@ -20,6 +20,7 @@
 #include "cbc_internal.h"
 #include "ensemble.h"
 #include "duo_core.cuh"
+#include "solo_core.cuh"
 #include "wide_core.cuh"
 
 namespace cbc {
@@ -106,7 +107,7 @@ __device__ __forceinline__ void ens_write_scalars(const EnsLayout& E, const Para
                     S.c->conv_fail, S.c->lin_iters);
 }
 
-// ---- 1 to 8 bubbles, and the direct solve for any number (ckm1d_core.cuh) ----
+// ---- 2 to 8 bubbles, and the direct solve for any number (ckm1d_core.cuh) ----
 
 // Loads system s into this lane's slot (lane li of the group) and runs the
 // prologue.  Called only by lanes whose group claimed s.
@@ -379,6 +380,95 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
   ensemble_worker(f, E, P, order, begin, end, head, max_steps, steps_total, epoch, budget_ns);
 }
 
+// The same for a single bubble per system with the Richardson solve: one system
+// per lane (solo_core.cuh).  slots: lanes of a warp that take systems.
+template <int KC>
+__global__ void __launch_bounds__(SOLO_THREADS, SOLO_BLOCKS)
+    ensemble_solo_kernel(EnsLayout E, Params P, const int* __restrict__ order, int begin, int end, int* head,
+                         long long max_steps, int steps_total, const long long* epoch, long long budget_ns,
+                         int slots) {
+  extern __shared__ __align__(16) double smem[];
+  const SoloSmem W = solo_smem(smem, P.nk);
+  const int lane = threadIdx.x & 31;
+  BubbleState S;
+  S.c = W.cold + lane;
+  S.o = W.own + lane;
+  S.lead = true;
+  S.active = false;
+  S.status = ST_ACTIVE;
+  int sys = -1;           // system of this lane (-1: none)
+  bool drained = lane >= slots;
+  const long long deadline = budget_ns > 0 ? epoch[0] + budget_ns : 0;
+
+  while (true) {
+    // time slice over: stop every system after its current step, claim no more
+    if (deadline != 0) {
+      long long now = 0;
+      if (lane == 0) now = global_ns();
+      now = __shfl_sync(FULL, now, 0);
+      if (now >= deadline) {
+        drained = true;
+        if (S.active) {
+          S.status = ST_MAX_STEPS;
+          S.active = false;
+        }
+      }
+    }
+    // retire finished systems and refill empty lanes
+    if (__any_sync(FULL, !S.active & !(sys < 0 & drained))) {
+      if (sys >= 0 && !S.active) {
+        ens_write_state(E, S.c->boff, S.y);
+        ens_write_scalars(E, P, sys, S);
+        sys = -1;
+      }
+      const bool want = sys < 0 && !drained;
+      const unsigned wmask = __ballot_sync(FULL, want);
+      if (wmask) {
+        int base_idx = 0;
+        if (lane == 0) base_idx = atomicAdd(head, __popc(wmask));
+        base_idx = __shfl_sync(FULL, base_idx, 0);
+        if (want) {
+          const int idx = begin + base_idx + __popc(wmask & ((1u << lane) - 1u));
+          if (idx < end) {
+            sys = order[idx];
+            const long long row = E.bubble_offset[sys];
+            if (E.trace_load_ns) E.trace_load_ns[sys] = global_ns();
+            ens_load_scalars(E, P, sys, S);
+            ens_load_state(E, row, S.y);
+            solo_store_bubble(W, lane, E.unit_params + row * E.up_stride, 1);
+            const double* sp = E.system_params + (long long)sys * E.sp_stride;
+            store_harmonics(W.hc + lane, 32, sp[1], sp[2], sp[4], E.control_params + (long long)sys * E.cp_stride,
+                            P.nk, 1);
+            ens_step_base(E, sys, steps_total, max_steps, S);
+            // first dense sample and initial event value
+            if (first_sample(S, P)) {
+              ens_store_dense(E, S.t, S.y, S.c->boff, 0, sys, S.o->idx);
+              first_stored(S, P);
+            }
+            if (S.active) S.g_old = 1e30;
+          } else {
+            drained = true;
+          }
+        }
+      }
+      __syncwarp();
+      if (!__any_sync(FULL, S.active)) {
+        if (!__any_sync(FULL, sys >= 0 || !drained)) break;
+        continue;
+      }
+      // systems that arrived already finished are written back by the next turn
+    }
+    // one Cash-Karp step for every active lane
+    const bool stq = solo_step(P, W, lane, S);
+    if (stq) ens_store_dense(E, S.t, S.y, S.c->boff, 0, sys, S.o->idx);
+    after_store(S, P, stq);
+    if (S.active && S.o->steps + S.c->step_base >= max_steps) {
+      S.status = ST_MAX_STEPS;
+      S.active = false;
+    }
+  }
+}
+
 // The same for 17 to 32 bubbles per system with the Richardson solve: one system
 // per block of two warps (duo_core.cuh).  KC: exact K, or 0 (read at run time).
 template <int KC>
@@ -484,7 +574,13 @@ cudaError_t launch_ensemble_k(const EnsLayout& E, const Params& P, const int* or
       constexpr int LIN = decltype(lin)::value, MB = KB <= 8 ? decltype(mbv)::value : 0;
       size_t shmem = kernel_smem(K, P.nk, LIN, threads);
       if (smem_bytes > shmem) shmem = smem_bytes;
-      if constexpr (KB == 32 && LIN == LIN_RICHARDSON) {
+      if constexpr (KC == 1 && LIN == LIN_RICHARDSON) {
+        const auto kernel = ensemble_solo_kernel<KC>;
+        const cudaError_t e = configure_kernel(kernel, shmem);
+        if (e != cudaSuccess) return e;
+        kernel<<<blocks, threads, shmem, stream>>>(E, P, order, begin, end, head, max_steps, steps_total, epoch,
+                                                   budget_ns, slots);
+      } else if constexpr (KB == 32 && LIN == LIN_RICHARDSON) {
         const auto kernel = ensemble_duo_kernel<KC>;
         const cudaError_t e = configure_kernel(kernel, shmem);
         if (e != cudaSuccess) return e;
@@ -514,7 +610,11 @@ cudaError_t occupancy_k(int K, int nk, int threads, int lin, int mb, int* n) {
   return dispatch_lin(lin, [&](auto li) {
     return dispatch_mb(KB <= 8 ? mb : 0, [&](auto mbv) {
       constexpr int LIN = decltype(li)::value, MB = KB <= 8 ? decltype(mbv)::value : 0;
-      if constexpr (KB == 32 && LIN == LIN_RICHARDSON) {
+      if constexpr (KC == 1 && LIN == LIN_RICHARDSON) {
+        const auto kernel = ensemble_solo_kernel<KC>;
+        configure_kernel(kernel, shmem);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, threads, shmem);
+      } else if constexpr (KB == 32 && LIN == LIN_RICHARDSON) {
         const auto kernel = ensemble_duo_kernel<KC>;
         configure_kernel(kernel, shmem);
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, threads, shmem);

@@ -9,6 +9,7 @@
 #include "cbc_internal.h"
 #include "duo_core.cuh"
 #include "plain.h"
+#include "solo_core.cuh"
 #include "wide_core.cuh"
 
 namespace cbc {
@@ -100,7 +101,7 @@ __device__ __forceinline__ void ref_write_scalars(const RefLayout& L, const Para
                     S.c->conv_fail, S.c->lin_iters, active_counter);
 }
 
-// One lane per bubble: 1 to 8 bubbles, and the direct solve (ckm1d_core.cuh).
+// One lane per bubble: 2 to 8 bubbles, and the direct solve (ckm1d_core.cuh).
 template <int KB, int KC, int LIN>
 __global__ void __launch_bounds__(128, min_blocks_for(KB))
     plain_kernel(RefLayout L, Params P, long long budget, int final_launch, int* active_counter) {
@@ -195,6 +196,47 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
   }
 }
 
+// The same for a single bubble per system with the Richardson solve: one system
+// per lane (solo_core.cuh).
+template <int KC>
+__global__ void __launch_bounds__(SOLO_THREADS, SOLO_BLOCKS)
+    plain_solo_kernel(RefLayout L, Params P, long long budget, int final_launch, int* active_counter) {
+  extern __shared__ __align__(16) double smem[];
+  const SoloSmem W = solo_smem(smem, P.nk);
+  const int lane = threadIdx.x & 31;
+  const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long NST = (long long)L.ns * L.tile;
+  const bool have = s < L.ns;
+  BubbleState S;
+  S.c = W.cold + lane;
+  S.o = W.own + lane;
+  S.lead = true;
+  S.active = false;
+  S.status = ST_ACTIVE;
+  if (have) {
+    ref_load(L, P, s, S);
+    ref_load_state(L, s * L.tile, S.y);
+    solo_store_bubble(W, lane, L.unit_params + s * L.tile, NST);
+    ref_store_harmonics(L, P, s, W.hc + lane, 32);
+    if (first_sample(S, P)) {
+      ref_store_dense(L, S.t, S.y, 0, s, S.o->idx);
+      first_stored(S, P);
+    }
+    if (S.active) S.g_old = 1e30;
+  }
+  for (long long it = 0; it < budget; ++it) {
+    if (!__any_sync(FULL, S.active)) break;
+    const bool st = solo_step(P, W, lane, S);
+    if (st) ref_store_dense(L, S.t, S.y, 0, s, S.o->idx);
+    after_store(S, P, st);
+  }
+  if (have) {
+    if (S.status == ST_ACTIVE && final_launch) S.status = ST_MAX_STEPS;
+    ref_write_state(L, S.y, s * L.tile);
+    ref_write_scalars(L, P, s, S, active_counter);
+  }
+}
+
 // The same for 17 to 32 bubbles per system with the Richardson solve: one system
 // per block of two warps (duo_core.cuh).
 template <int KC>
@@ -260,7 +302,8 @@ cudaError_t launch_plain_k(const RefLayout& L, const Params& P, long long budget
       kernel<<<(unsigned)blocks, threads, shmem, stream>>>(L, P, budget, final_launch, counter);
       return cudaGetLastError();
     };
-    if constexpr (KB == 16 && LIN == LIN_RICHARDSON) return launch(plain_wide_kernel<KC>);
+    if constexpr (KC == 1 && LIN == LIN_RICHARDSON) return launch(plain_solo_kernel<KC>);
+    else if constexpr (KB == 16 && LIN == LIN_RICHARDSON) return launch(plain_wide_kernel<KC>);
     else if constexpr (KB == 32 && LIN == LIN_RICHARDSON) return launch(plain_duo_kernel<KC>);
     else return launch(plain_kernel<KB, KC, LIN>);
   });
