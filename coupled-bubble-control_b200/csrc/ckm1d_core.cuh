@@ -41,7 +41,7 @@
 #include <stdint.h>
 #include <string.h>
 #include <utility>
-#include "cbc_math.h"
+#include "cbc_math_dev.cuh"
 
 namespace cbc {
 
@@ -238,6 +238,7 @@ struct LaneState {
   int idx;                     // dense samples stored
   int status;
   bool active;
+  bool normal;                 // constants and phases within the range of the fast functions
   int steps, rejected, conv_ok, conv_fail;
   long long lin_iters;
 };
@@ -576,14 +577,80 @@ __device__ __forceinline__ void lu_solve_smem(const Geo& g, const WarpSmem& W, d
   xt = W.mat[(srcT >= K ? RS * 32 : 0) + N * 32 + oT] * rpT;
 }
 
+// Elementary functions of a right-hand side: the branch-free forms for the normal
+// range (FAST) or the general ones.  Same values.
+template <bool FAST>
+__device__ __forceinline__ double f_rcp(double x) {
+  if constexpr (FAST) {
+    double y[1];
+    cbcd::rcp<1>({x}, y);
+    return y[0];
+  } else {
+    return 1.0 / x;
+  }
+}
+template <bool FAST>
+__device__ __forceinline__ double f_pow(double x, double y) {
+  if constexpr (FAST) {
+    double out[1];
+    cbcd::pow_pos<1>({x}, {y}, out);
+    return out[0];
+  } else {
+    return cbcm::pow_pos(x, y);
+  }
+}
+template <bool FAST>
+__device__ __forceinline__ void f_sincos(double x, double* s, double* c) {
+  if constexpr (FAST) {
+    double a[1], b[1];
+    cbcd::sincos<1>({x}, a, b);
+    *s = a[0];
+    *c = b[0];
+  } else {
+    cbcm::sincos(x, s, c);
+  }
+}
+
+// Range of the FAST forms.  Constants and phases of a system, tested once when
+// it is loaded (sp0, sp1, sp2: system parameters; cp[m cp_stride]: control
+// parameters as in store_harmonics): 3 gamma <= 15, phases below 2^50 up to
+// t_end and for positions below 2^32.
+__device__ __forceinline__ int system_in_range(double sp0, double sp1, double sp2, const double* cp, int nk,
+                                               long long cp_stride, double t, double t_end) {
+  const double tm = fabs(t) > fabs(t_end) ? fabs(t) : fabs(t_end);
+  bool ok = fabs(sp0) <= 15.0;
+  for (int k = 0; k < nk; ++k) {
+    const double omega = cp[(nk + k) * cp_stride], phase = cp[(2 * nk + k) * cp_stride],
+                 wave = cp[(3 * nk + k) * cp_stride];
+    ok = ok && fma(fabs(TWO_PI * sp1 * omega), tm, fabs(phase)) < 0x1p50 && fabs(TWO_PI * sp2 * wave) < 0x1p17;
+  }
+  return ok ? 1 : 0;
+}
+// Arguments of one evaluation: radius (dimensionless) in [2^-64, 2^64), so
+// that |3 gamma log R| < 690; position below 2^32 (so pair distances are at
+// most 2^33); the Keller--Miksis denominator D in [2^-500, 2^500).  Physical
+// states are far inside; a state that is about to fail (a singular
+// denominator, an overflow) takes the general functions, with the same values.
+__device__ __forceinline__ bool state_in_range(double x0, double x1, double D) {
+  return (x0 > 0.0) & cbcd::exp_in<-64, 64>(x0) &
+         ((unsigned)(__double2hiint(x1) & 0x7fffffff) < (unsigned)((1023 + 32) << 20)) & cbcd::exp_in<-500, 500>(D);
+}
+
 // Right-hand side for one field form: NKC harmonics and field type ACC
 // known at compile time (NKC = 0, ACC = -1: both read from P).  With both
 // fixed the harmonic loops have no branches, so the independent sin/cos,
 // log/exp and division chains of the bubble interleave.
-template <int KB, int KC, int LIN, int NKC, int ACC>
+// FAST: reciprocals and elementary functions without branches, for arguments in
+// the range that in_range reports (state_in_range); the caller evaluates an attempt
+// again without FAST if some argument was outside.  A compiler reciprocal ends in
+// a branch, as the special cases of the general functions do: the seven of a
+// K = 8 bubble's partners took 74 cycles each, one after the other.  A step attempt
+// before and after: K = 2 alone 13.6 us, now 11.1, K = 4 17.9, 15.5, K = 8 26.0,
+// 22.0; GPU full K = 2 0.650 ns, 0.630, K = 8 7.69, 7.23.
+template <int KB, int KC, int LIN, int NKC, int ACC, bool FAST>
 __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const WarpSmem& W,
                                          double sp0, double sp3, bool on, double t, const double y[4],
-                                         double dy[4], bool& conv, int& iters) {
+                                         double dy[4], bool& in_range, bool& conv, int& iters) {
   const int nk = NKC > 0 ? NKC : P.nk;
   const int ac = ACC >= 0 ? ACC : P.ac;
   const int K = g.K;
@@ -595,7 +662,7 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
   if (nk <= K) {
     const int k = li < nk ? li : 0;
     double s_, c_;
-    cbcm::sincos(fma(hcv(W, g, k, 0), t, hcv(W, g, k, 1)), &s_, &c_);
+    f_sincos<FAST>(fma(hcv(W, g, k, 0), t, hcv(W, g, k, 1)), &s_, &c_);
 #pragma unroll
     for (int kk = 0; kk < NKMAX; ++kk)
       if (kk < nk) {
@@ -605,12 +672,12 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
   } else {
 #pragma unroll
     for (int kk = 0; kk < NKMAX; ++kk)
-      if (kk < nk) cbcm::sincos(fma(hcv(W, g, kk, 0), t, hcv(W, g, kk, 1)), &st[kk], &ct[kk]);
+      if (kk < nk) f_sincos<FAST>(fma(hcv(W, g, kk, 0), t, hcv(W, g, kk, 1)), &st[kk], &ct[kk]);
   }
 
   // ---- uncoupled Keller--Miksis + translation (ckm1d_def.py:418-447) ----
-  const double rx0 = 1.0 / x0;
-  const double p = cbcm::pow_pos(rx0, sp0);
+  const double rx0 = f_rcp<FAST>(x0);
+  const double p = f_pow<FAST>(rx0, sp0);
   double pa = 0.0, pt = 0.0, px = 0.0, ux = 0.0;
 #pragma unroll
   for (int k = 0; k < NKMAX; ++k) {
@@ -621,7 +688,7 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
         pt = fma(aw, ct[k], pt);
       } else {
         double sx, cx;
-        cbcm::sincos(fma(hcv(W, g, k, 2), x1, hcv(W, g, k, 1)), &sx, &cx);
+        f_sincos<FAST>(fma(hcv(W, g, k, 2), x1, hcv(W, g, k, 1)), &sx, &cx);
         const double awv = hcv(W, g, k, 5), au = hcv(W, g, k, 6);
         if (ac == 1) {  // SW_N
           pa = fma(a * sx, st[k], pa);
@@ -681,7 +748,7 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
         const double delta = x1 - xj1;
         const double sg = (double)((delta > 0.0) - (delta < 0.0));
         const double ad = fabs(delta);
-        const double rd = 1.0 / (ad > 1e-30 ? ad : 1e-30);
+        const double rd = f_rcp<FAST>(ad > 1e-30 ? ad : 1e-30);
         const double rd2 = rd * rd;
         const double srd2 = rd2 * sg;
         const double rd3 = rd2 * rd;
@@ -738,7 +805,8 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
   N = fma(-(upv(W, g, 6) * pt), x0, N);
   N = fma(upv(W, g, 8) * x3, x3, N);
   const double D = fma(-(u7 * x0), x2, x0) + upv(W, g, 14);
-  const double rD = 1.0 / D;
+  const double rD = f_rcp<FAST>(D);
+  in_range = !FAST || state_in_range(x0, x1, D);
   const double x02 = x0 * x0;
   const double x03 = x02 * x0;
   const double Fb1 = -(upv(W, g, 10) * x03) * px;
@@ -850,22 +918,6 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
   dy[3] = vt;
 }
 
-// Field forms with their own compiled right-hand side: two harmonics of a
-// standing wave with the antinode (SW_A) or the node (SW_N) at x = 0, the
-// forms of the benchmarked workloads; any other form uses the general one.
-// P is uniform over a launch, so the branch never diverges.
-template <int KB, int KC, int LIN>
-__device__ __forceinline__ void rhs(const Geo& g, const Params& P, const WarpSmem& W,
-                                    double sp0, double sp3, bool on, double t, const double y[4],
-                                    double dy[4], bool& conv, int& iters) {
-  if (P.nk == 2 && P.ac == 2)
-    rhs_form<KB, KC, LIN, 2, 2>(g, P, W, sp0, sp3, on, t, y, dy, conv, iters);
-  else if (P.nk == 2 && P.ac == 1)
-    rhs_form<KB, KC, LIN, 2, 1>(g, P, W, sp0, sp3, on, t, y, dy, conv, iters);
-  else
-    rhs_form<KB, KC, LIN, 0, -1>(g, P, W, sp0, sp3, on, t, y, dy, conv, iters);
-}
-
 // Exact sample time k of the grid dense mode.
 __device__ __forceinline__ double grid_time(const LaneState& S, int k, int ndo) {
   if (k >= ndo - 1 && ndo > 1) return S.t_end;
@@ -948,38 +1000,57 @@ __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSm
   }
   const double t = S.t;
   double* ks = W.ks + g.lane;   // ks[(st * 4 + c) * 32]
-  int conv_fail_here = 0;
 
-  // six Cash-Karp stages (stepper.py:379-480), one RHS call site
+  // six Cash-Karp stages (stepper.py:379-480).  Field forms with their own
+  // compiled right-hand side: two harmonics of a standing wave with the antinode
+  // (SW_A) or the node (SW_N) at x = 0, the forms of the benchmarked workloads;
+  // any other form uses the general one (P is uniform over a launch, so the
+  // branch never diverges), and so does an attempt in which some argument of the
+  // warp was outside the range of the fast functions: it is evaluated again.
+  constexpr bool FAST = LIN == LIN_RICHARDSON;
+  bool general = P.nk != 2 || P.ac == 0;
+  int conv_fail_here, sweeps;
+  while (true) {
+    bool in_range = true;
+    conv_fail_here = sweeps = 0;
 #pragma unroll 1
-  for (int st = 0; st < 6; ++st) {
-    double ys[4];
-    switch (st) {
-      case 0:
+    for (int st = 0; st < 6; ++st) {
+      double ys[4];
+      switch (st) {
+        case 0:
 #pragma unroll
-        for (int c = 0; c < 4; ++c) ys[c] = S.y[c];
-        break;
-      case 1: stage_state<1>(ks, h, S.y, ys); break;
-      case 2: stage_state<2>(ks, h, S.y, ys); break;
-      case 3: stage_state<3>(ks, h, S.y, ys); break;
-      case 4: stage_state<4>(ks, h, S.y, ys); break;
-      default: stage_state<5>(ks, h, S.y, ys); break;
-    }
-    const double ts = (st == 0) ? t : fma(kStageA[st], h, t);
-    double kk[4];
-    bool cv;
-    int it;
-    rhs<KB, KC, LIN>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, cv, it);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) ks[(st * 4 + c) * 32] = kk[c];
-    if (on) {
-      S.lin_iters += it;
-      if (cv) ++S.conv_ok;
-      else {
-        ++S.conv_fail;
-        ++conv_fail_here;
+          for (int c = 0; c < 4; ++c) ys[c] = S.y[c];
+          break;
+        case 1: stage_state<1>(ks, h, S.y, ys); break;
+        case 2: stage_state<2>(ks, h, S.y, ys); break;
+        case 3: stage_state<3>(ks, h, S.y, ys); break;
+        case 4: stage_state<4>(ks, h, S.y, ys); break;
+        default: stage_state<5>(ks, h, S.y, ys); break;
       }
+      const double ts = (st == 0) ? t : fma(kStageA[st], h, t);
+      double kk[4];
+      bool cv, ok;
+      int it;
+      if (!general && P.ac == 2)
+        rhs_form<KB, KC, LIN, 2, 2, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
+      else if (!general)
+        rhs_form<KB, KC, LIN, 2, 1, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
+      else
+        rhs_form<KB, KC, LIN, 0, -1, false>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) ks[(st * 4 + c) * 32] = kk[c];
+      in_range = in_range & ok;
+      sweeps += it;
+      conv_fail_here += cv ? 0 : 1;
     }
+    if (!FAST || general) break;
+    if (__all_sync(FULL, !on | (in_range & S.normal))) break;
+    general = true;
+  }
+  if (on) {
+    S.lin_iters += sweeps;
+    S.conv_ok += 6 - conv_fail_here;
+    S.conv_fail += conv_fail_here;
   }
 
   // candidate (c2 = c5 = 0) and embedded error estimate (ce2 = 0)

@@ -5,7 +5,6 @@
 // Same operations in the same order as ckm1d_core.cuh.
 #pragma once
 
-#include "cbc_math_dev.cuh"
 #include "ckm1d_core.cuh"
 
 namespace cbc {
@@ -99,31 +98,6 @@ __device__ __forceinline__ PairTerms pair_terms(const PartnerTerms& q, double rd
   p.c = -((m1 * srd2) * q.j02);
   p.d = -((m1 * rd3) * q.j03);
   return p;
-}
-
-// Range of the FAST forms.  Constants and phases of a system, tested once when
-// it is loaded (sp0, sp1, sp2: system parameters; cp[m cp_stride]: control
-// parameters as in store_harmonics): 3 gamma <= 15, phases below 2^50 up to
-// t_end and for positions below 2^32.
-__device__ __forceinline__ int system_in_range(double sp0, double sp1, double sp2, const double* cp, int nk,
-                                               long long cp_stride, double t, double t_end) {
-  const double tm = fabs(t) > fabs(t_end) ? fabs(t) : fabs(t_end);
-  bool ok = fabs(sp0) <= 15.0;
-  for (int k = 0; k < nk; ++k) {
-    const double omega = cp[(nk + k) * cp_stride], phase = cp[(2 * nk + k) * cp_stride],
-                 wave = cp[(3 * nk + k) * cp_stride];
-    ok = ok && fma(fabs(TWO_PI * sp1 * omega), tm, fabs(phase)) < 0x1p50 && fabs(TWO_PI * sp2 * wave) < 0x1p17;
-  }
-  return ok ? 1 : 0;
-}
-// Arguments of one evaluation: radius (dimensionless) in [2^-64, 2^64), so
-// that |3 gamma log R| < 690; position below 2^32 (so pair distances are at
-// most 2^33); the Keller--Miksis denominator D in [2^-500, 2^500).  Physical
-// states are far inside; a state that is about to fail (a singular
-// denominator, an overflow) takes the general functions, with the same values.
-__device__ __forceinline__ bool state_in_range(double x0, double x1, double D) {
-  return (x0 > 0.0) & cbcd::exp_in<-64, 64>(x0) &
-         ((unsigned)(__double2hiint(x1) & 0x7fffffff) < (unsigned)((1023 + 32) << 20)) & cbcd::exp_in<-500, 500>(D);
 }
 
 // Elementary functions of several arguments, interleaved (FAST) or one after the

@@ -126,6 +126,8 @@ __device__ __forceinline__ void lane_load(const EnsLayout& E, const Params& P, c
   S.t_begin = E.t_begin[s];
   S.h = E.h[s];
   S.idx = (P.ndo > 0) ? E.dense_index[s] : 0;
+  S.normal = system_in_range(sp[0], sp[1], sp[2], E.control_params + (long long)s * E.cp_stride, P.nk, 1, S.t,
+                             S.t_end) != 0;
   prologue(S, P, E.event[s], ens_prev_time(E, P, s, S.idx), E.status[s]);
   store_coupling(W, g, MView{E.coupling + E.coupling_offset[s] + g.li, (long long)g.K * g.K, g.K});
   if (g.li == 0) store_harmonics(W.hc + g.grp, g.G, sp[1], sp[2], sp[4], E.control_params + (long long)s * E.cp_stride, P.nk, 1);

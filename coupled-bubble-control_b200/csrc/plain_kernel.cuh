@@ -52,6 +52,7 @@ __device__ __forceinline__ void ref_load(const RefLayout& L, const Params& P, lo
   S.t_begin = L.time_begin[s];
   S.h = L.time_step[s];
   S.idx = (P.ndo > 0) ? L.dense_index[s] : 0;
+  S.normal = ref_in_range(L, P, s, S.t, S.t_end) != 0;
   prologue(S, P, L.actual_event[s], ref_prev_time(L, P, s, S.idx), L.status[s]);
 }
 __device__ __forceinline__ void ref_load(const RefLayout& L, const Params& P, long long s, ScalarState& S) {

@@ -18,7 +18,7 @@ from test_parity_ensemble import compare, oracle_ragged
 
 pytestmark = pytest.mark.gpu
 
-FORMS = [1, 9, 11, 15, 16, 17, 24, 31, 32]
+FORMS = [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 15, 16, 17, 24, 31, 32]
 FIELDS = [("SW_A", 2), ("SW_N", 2), ("CONST", 2), ("SW_A", 1), ("SW_N", 3), ("SW_A", 4)]
 
 
