@@ -9,10 +9,6 @@
 
 namespace cbc {
 
-// Weights of k1, k3, k4, k5, k6 in the candidate (k5: 0) and in the error estimate.
-static __constant__ double kC[5] = {C1, C3, C4, 0.0, C6};
-static __constant__ double kCE[5] = {CE1, CE3, CE4, CE5, CE6};
-
 // Scalars of a system that an attempt touches once or not at all: kept in
 // shared memory, so that they take no registers inside the right-hand side.
 // One record per system: written when the system is loaded, then read by all its
@@ -341,43 +337,6 @@ __device__ __forceinline__ double attempt_step(const ScalarState& S, const Param
     }
   }
   return h;
-}
-
-// Candidate (c2 = c5 = 0) and embedded error estimate (ce2 = 0) of one bubble
-// from k1..k5 in ks and k6: its finiteness, acceptance and smallest
-// tolerance / error ratio.
-__device__ __forceinline__ void candidate(const Params& P, bool on, double h, const double y[4], const double* ks, int stride,
-                                          const double k6[4], double yn[4], bool& fin, bool& ok, double& ratio) {
-  double tol[4], e[4], r[4];
-  bool normal = true;
-  fin = ok = true;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const double k1 = ks[c * stride], k3 = ks[(8 + c) * stride], k4 = ks[(12 + c) * stride], k5 = ks[(16 + c) * stride];
-    const double acc = fma(kC[4], k6[c], fma(kC[2], k4, fma(kC[1], k3, kC[0] * k1)));
-    yn[c] = fma(h, acc, y[c]);
-    fin = fin & cbcm::isfinite_(yn[c]);
-    const double es = fma(kCE[4], k6[c], fma(kCE[3], k5, fma(kCE[2], k4, fma(kCE[1], k3, kCE[0] * k1))));
-    e[c] = fabs(h * es) + 1.0e-18;
-    const double ay = fabs(yn[c]), ao = fabs(y[c]);
-    const double tl = P.rtol * (ay > ao ? ay : ao);
-    tol[c] = tl > P.atol ? tl : P.atol;
-    normal = normal & cbcd::exp_in<-400, 400>(e[c]) & cbcd::exp_in<-400, 400>(tol[c]);
-  }
-  cbcd::quot(tol, e, r);
-  if (on & !normal) {     // (idle lanes hold anything)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) r[c] = tol[c] / e[c];
-  }
-  // smallest ratio below 1e30, NaN ignored
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    ok = ok & !(r[c] < 1.0);
-    r[c] = r[c] < 1.0e30 ? r[c] : 1.0e30;
-  }
-  r[0] = r[1] < r[0] ? r[1] : r[0];
-  r[2] = r[3] < r[2] ? r[3] : r[2];
-  ratio = r[2] < r[0] ? r[2] : r[0];
 }
 
 // Controller, acceptance and dense-output decision after an attempt

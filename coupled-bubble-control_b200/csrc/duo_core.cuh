@@ -332,7 +332,7 @@ __device__ __forceinline__ bool duo_step(const DuoGeo& g, const Params& P, const
   }
   double yn[4], ratio;
   bool fin, ok;
-  candidate(P, g.valid, h, S.y, ks, 32, kk, yn, fin, ok, ratio);
+  candidate<true>(P, g.valid, h, S.y, ks, 32, kk, yn, fin, ok, ratio);
   const double g_new = duo_event(g, W, yn, P.col, fin, ok, ratio);
   count_attempt(S, sweeps, conv_fail_here);
   bool accepted;

@@ -124,7 +124,7 @@ __device__ __forceinline__ bool solo_step(const Params& P, const SoloSmem& W, in
   }
   double yn[4], ratio;
   bool fin, okerr;
-  candidate(P, on, h, S.y, ks, 32, kk, yn, fin, okerr, ratio);
+  candidate<true>(P, on, h, S.y, ks, 32, kk, yn, fin, okerr, ratio);
   if (!on) return false;
   count_attempt(S, sweeps, conv_fail_here);
   bool accepted;

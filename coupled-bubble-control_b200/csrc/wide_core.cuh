@@ -273,7 +273,7 @@ __device__ __forceinline__ bool wide_step(const Geo& g, const Params& P, const W
   }
   double yn[4], ratio_l;
   bool fin, ok_l;
-  candidate(P, on, h, S.y, ks, 32, kk, yn, fin, ok_l, ratio_l);
+  candidate<true>(P, on, h, S.y, ks, 32, kk, yn, fin, ok_l, ratio_l);
   const bool finite = group_all(fin, g);
   const double g_new = group_event<WIDE>(yn, upv(W, g, 12), g, P.col);
   const double ratio = group_min<WIDE>(ratio_l, g);
