@@ -353,21 +353,45 @@ __device__ __forceinline__ double group_sum_full(double v) {
   return v;
 }
 
+// How the Richardson iterates reach a lane's partners: by two 64-bit shuffles a
+// partner, or through the partner-state records (free by then), one 8-byte store
+// and K - 1 loads per value, in two buffers used in turn so that a sweep needs
+// one __syncwarp.  Cycles a sweep of one warp, shuffled / stored (measured):
+// K = 2: 74 / 83, 3: 99 / 112, 4: 120 / 114, 5: 145 / 169, 6: 166 / 188,
+// 7: 188 / 211, 8: 215 / 178.  Eight bubbles: an attempt alone 21.1 us shuffled, 20.1
+// stored, GPU full 7.18 ns, 6.71.  Four: alone 14.6 us, 14.3, but GPU full 1.98 ns,
+// 2.06 (so shuffled).
+__host__ __device__ constexpr bool iterates_stored(int K) { return K == 8; }
+
 // Residual r = b - A v of the implicit coupling system for this lane's bubble,
 // A = I + off-diagonal partner blocks.  Partner distance d = 1..K-1 goes to
 // accumulation chain (d - 1) mod 4 (increasing d within a chain); the chains
 // accumulation chain (d - 1) mod 4 (increasing d within a chain); the chains
 // are then combined by the open pairwise tree.
-template <int KB>
-__device__ __forceinline__ void residual(const Geo& g, const double* Am, const double* Bm, const double* Cm,
-                                         const double* Dm, double cpf0, double b0, double b1, double vr,
-                                         double vt, double& r0, double& r1) {
+template <int KB, int KC>
+__device__ __forceinline__ void residual(const Geo& g, const WarpSmem& W, int buf, const double* Am, const double* Bm,
+                                         const double* Cm, const double* Dm, double cpf0, double b0, double b1,
+                                         double vr, double vt, double& r0, double& r1) {
   double ar[4] = {0.0, 0.0, 0.0, 0.0}, at[4] = {0.0, 0.0, 0.0, 0.0};
+  double* x = W.xv + 64 * buf;
+  if constexpr (iterates_stored(KC)) {
+    x[g.lane] = vr;
+    x[32 + g.lane] = vt;
+    __syncwarp();
+  }
 #pragma unroll
   for (int d = 1; d < KB; ++d)
     if (d < g.K) {
-      const int src = partner_lane(g, d);
-      const double vrj = shfl(vr, src), vtj = shfl(vt, src);
+      double vrj, vtj;
+      if constexpr (iterates_stored(KC)) {
+        const int src = partner_rec(g, d);
+        vrj = x[src];
+        vtj = x[32 + src];
+      } else {
+        const int src = partner_lane(g, d);
+        vrj = shfl(vr, src);
+        vtj = shfl(vt, src);
+      }
       const int c = (d - 1) & 3;
       ar[c] = fma(Am[d], vrj, fma(Bm[d], vtj, ar[c]));
       at[c] = fma(Cm[d], vrj, fma(Dm[d], vtj, at[c]));
@@ -870,17 +894,18 @@ __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const Wa
   const bool full_groups = (g.K == KB);
   const int maxit = P.lin_max_iter;
   double r0, r1;
-  residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, vr, vt, r0, r1);
+  if constexpr (iterates_stored(KC)) __syncwarp();   // every lane has read its partners' states
+  residual<KB, KC>(g, W, 1, Am, Bm, Cm, Dm, cpf0, b0, b1, vr, vt, r0, r1);
   for (int it = 0; it < maxit; it += 2) {
     if (__all_sync(FULL, found)) break;
     // iterate it: (vr, vt) with residual (r0, r1); iterate it + 1: (br, bt)
     const double br = fma(P.omega, r0, vr), bt = fma(P.omega, r1, vt);
     double q0, q1;
-    residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, br, bt, q0, q1);
+    residual<KB, KC>(g, W, 0, Am, Bm, Cm, Dm, cpf0, b0, b1, br, bt, q0, q1);
     const bool two = it + 1 < maxit;   // the plain loop also tests iterate it + 1
     const double wr = fma(P.omega, q0, br), wt = fma(P.omega, q1, bt);
     double s0, s1;
-    residual<KB>(g, Am, Bm, Cm, Dm, cpf0, b0, b1, wr, wt, s0, s1);
+    residual<KB, KC>(g, W, 1, Am, Bm, Cm, Dm, cpf0, b0, b1, wr, wt, s0, s1);
     const double rra = fma(r0, r0, r1 * r1), rrb = fma(q0, q0, q1 * q1);
     double rna, rnb;
     if (full_groups) {
