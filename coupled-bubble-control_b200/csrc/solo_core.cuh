@@ -68,7 +68,8 @@ __device__ __forceinline__ void solo_rhs_form(const Params& P, const SoloSmem& W
   double vr = b0, vt = b1;
   bool found = !on;
   iters = 0;
-  for (int it = 0; it < P.lin_max_iter && !__all_sync(FULL, found); ++it) {
+  for (int it = 0; it < P.lin_max_iter; ++it) {
+    if (__all_sync(FULL, found)) break;
     const double r0 = b0 - fma(0.0, o.rD, vr), r1 = b1 - (0.0 + vt);
     iters = found ? iters : it + 1;
     found = found | (fma(r0, r0, r1 * r1) < tol2);
@@ -120,7 +121,8 @@ __device__ __forceinline__ bool solo_step(const Params& P, const SoloSmem& W, in
       sweeps += it;
       conv_fail_here += cv ? 0 : 1;
     }
-    if (general || __all_sync(FULL, !on | in_range)) break;
+    if (general) break;
+    if (__all_sync(FULL, !on | in_range)) break;
   }
   double yn[4], ratio;
   bool fin, okerr;
