@@ -21,6 +21,7 @@
 #include "ensemble.h"
 #include "duo_core.cuh"
 #include "solo_core.cuh"
+#include "warp_turn.h"
 #include "wide_core.cuh"
 
 namespace cbc {
@@ -416,8 +417,12 @@ __global__ void __launch_bounds__(SOLO_THREADS, SOLO_BLOCKS)
         }
       }
     }
+    const unsigned active = __ballot_sync(FULL, S.active), held = __ballot_sync(FULL, sys >= 0),
+                   done = __ballot_sync(FULL, drained);
+    const Turn turn = next_turn(active, held, done);
+    if (turn == Turn::exit) break;
     // retire finished systems and refill empty lanes
-    if (__any_sync(FULL, !S.active & !(sys < 0 & drained))) {
+    if (turn == Turn::refill) {
       if (sys >= 0 && !S.active) {
         ens_write_state(E, S.c->boff, S.y);
         ens_write_scalars(E, P, sys, S);
@@ -454,11 +459,7 @@ __global__ void __launch_bounds__(SOLO_THREADS, SOLO_BLOCKS)
         }
       }
       __syncwarp();
-      if (!__any_sync(FULL, S.active)) {
-        if (!__any_sync(FULL, sys >= 0 || !drained)) break;
-        continue;
-      }
-      // systems that arrived already finished are written back by the next turn
+      continue;    // systems that arrived already finished go straight back out
     }
     // one Cash-Karp step for every active lane
     const bool stq = solo_step(P, W, lane, S);
