@@ -110,8 +110,6 @@ static EnsLayout make_layout(const cbc_ensemble* e) {
 constexpr int kDefaultThreads = 128;
 constexpr float kStartFill = 0.85f;
 
-constexpr int kExclusiveThreads = 128;
-
 // Per-bucket launch parameters.  The storage is a template parameter so that
 // the allocation-free entry point can use fixed arrays (FixedVec) while the
 // others keep std::vector.
@@ -164,14 +162,8 @@ static G grid_sizes(cbc_context* ctx, const cbc_spec* spec, const cbc_work* w) {
     if (n < 1) continue;
     g.exclusive[b] = 1;
     g.first[b] = n;
-    g.threads[b] = block_threads_for(w->bucket_K[b], spec->nk, spec->lin_solver, max_block_smem(ctx->device),
-                                     kExclusiveThreads);
+    g.threads[b] = lane_threads_for(w->bucket_K[b], spec->nk, spec->lin_solver, max_block_smem(ctx->device));
     g.smem[b] = max_block_smem(ctx->device);
-    if (duo_form(w->bucket_K[b], spec->lin_solver)) {
-      // two-lane form: DUO_BLOCKS blocks of two warps fill the SM between them
-      g.first[b] = n * DUO_BLOCKS;
-      g.smem[b] = (g.smem[b] / DUO_BLOCKS - 1024) & ~(size_t)15;
-    }
     excl_sms += n;
   }
   const float rest = 1.f - (float)excl_sms / (float)ctx->sm_count;

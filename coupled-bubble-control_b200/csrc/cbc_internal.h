@@ -133,7 +133,7 @@ constexpr size_t kScheduleBytes = kHeadBytes + 2 * sizeof(long long);
 cudaError_t noalloc_scratch_address(int device, void** out);
 
 // Systems of this many bubbles and this solver run on the two-lane form
-// (duo_core.cuh): one system per block of DUO_THREADS threads.
+// (duo_core.cuh): one system per team of DUO_THREADS threads.
 inline bool duo_form(int K, int lin) { return K > 16 && lin == LIN_RICHARDSON; }
 
 // Of these on the one-lane form (solo_core.cuh): 32 systems per warp.
@@ -144,7 +144,7 @@ inline bool wide_form(int K, int lin) { return K > 8 && K <= 16 && lin == LIN_RI
 
 // Dynamic shared memory of a block of `threads` threads.
 inline size_t kernel_smem(int K, int nk, int lin, int threads) {
-  if (duo_form(K, lin)) return sizeof(double) * (size_t)duo_smem_doubles(nk);
+  if (duo_form(K, lin)) return sizeof(double) * (size_t)duo_smem_doubles(nk) * (threads / DUO_THREADS);
   const int warp = solo_form(K, lin)   ? solo_smem_doubles(nk)
                    : wide_form(K, lin) ? wide_smem_doubles(K, nk)
                                        : smem_doubles_per_warp(K, nk, lin);
@@ -163,9 +163,16 @@ inline int block_threads_for(int K, int nk, int lin, size_t max_block_smem, int 
   return warps * 32;
 }
 
+// Threads of a latency lane's block, which holds an SM alone: four warps, or as
+// many two-warp teams as the registers of an SM are for.
+inline int lane_threads_for(int K, int nk, int lin, size_t max_block_smem) {
+  if (duo_form(K, lin)) return DUO_THREADS * DUO_BLOCKS;
+  return block_threads_for(K, nk, lin, max_block_smem, 128);
+}
+
 // Systems a block holds at once; slots: at most this many per warp.
 inline int systems_per_block(int K, int lin, int threads, int slots) {
-  if (duo_form(K, lin)) return 1;
+  if (duo_form(K, lin)) return threads / DUO_THREADS;
   const int fit = solo_form(K, lin) ? 32 : 32 / K;
   return (fit < slots ? fit : slots) * (threads / 32);
 }

@@ -17,35 +17,70 @@
 // radial ones, lane 1 the three translational ones, each over all partners,
 // with the terms of the other lane's partners shuffled over), the pairwise tree of
 // the norms.  Every value that decides control flow is the same in all 64
-// threads, so the block needs no votes, only barriers around its exchanges.
+// threads, so the team needs no votes, only barriers around its exchanges.
 #pragma once
 
 #include "cold_core.cuh"
 
 namespace cbc {
 
-constexpr int DUO_THREADS = 64;
-constexpr int DUO_BLOCKS = 4;     // resident blocks per SM the registers are limited for
+constexpr int DUO_THREADS = 64;   // of a team: one system
+constexpr int DUO_BLOCKS = 4;     // teams per SM the registers are limited for
 
+// TEAMS: systems of a block.  One, or as many as an SM has registers for where
+// the block has to hold its SM alone (latency lanes: blocks of one team each are
+// spread over as many SMs, beside other buckets' work).  One lane SM with 6,000
+// systems of 8 bubbles on the others: an attempt of four systems of K = 32 66 us
+// each, of one 42; K = 20 72 and 56.
+template <int TEAMS>
 struct DuoGeo {
   int K;
-  int tid;
+  int tid;     // thread of the team
+  int team;
   int i;       // bubble of this thread
   int c;       // lane of the pair
   bool valid;  // i < K
 };
 
-__device__ __forceinline__ DuoGeo make_duo_geo(int K) {
-  DuoGeo g;
+template <int TEAMS>
+__device__ __forceinline__ DuoGeo<TEAMS> make_duo_geo(int K) {
+  DuoGeo<TEAMS> g;
   g.K = K;
-  g.tid = threadIdx.x;
-  g.i = threadIdx.x >> 1;
-  g.c = threadIdx.x & 1;
+  g.tid = TEAMS > 1 ? threadIdx.x % DUO_THREADS : threadIdx.x;
+  g.team = TEAMS > 1 ? threadIdx.x / DUO_THREADS : 0;
+  g.i = g.tid >> 1;
+  g.c = g.tid & 1;
   g.valid = g.i < K;
   return g;
 }
 
-// Shared memory of a block, in doubles.
+// Barrier of the team's two warps, and the same with an OR over their threads.
+template <int TEAMS>
+__device__ __forceinline__ void duo_sync(const DuoGeo<TEAMS>& g) {
+  if constexpr (TEAMS == 1) __syncthreads();
+  else asm volatile("barrier.sync %0, %1;" ::"r"(1 + g.team), "n"(DUO_THREADS) : "memory");
+}
+template <int TEAMS>
+__device__ __forceinline__ bool duo_sync_or(const DuoGeo<TEAMS>& g, bool v) {
+  if constexpr (TEAMS == 1) {
+    return __syncthreads_or(v) != 0;
+  } else {
+    int r;
+    asm volatile(
+        "{\n"
+        "  .reg .pred p, q;\n"
+        "  setp.ne.s32 p, %1, 0;\n"
+        "  barrier.red.or.pred q, %2, %3, p;\n"
+        "  selp.s32 %0, 1, 0, q;\n"
+        "}"
+        : "=r"(r)
+        : "r"((int)v), "r"(1 + g.team), "n"(DUO_THREADS)
+        : "memory");
+    return r != 0;
+  }
+}
+
+// Shared memory of a team, in doubles.
 struct DuoSmem {
   double* hc;    // [7 nk]    harmonic constants
   double* up;    // [13][32]  bubble constants
@@ -55,40 +90,45 @@ struct DuoSmem {
   double* rr;    // [2][32]   squared residuals
   double* cm;    // [3][32][32] coupling coefficients of partner d = 1..32 (zero past K - 1)
   double* red;   // [2][4]    per-warp results of the step's reductions
+  int* claim;    // [2]       claimed system; whether the time slice is over
   LaneCold* own; // [64]
   Cold* cold;    // scalars of the system
 };
 
 __host__ __device__ inline int duo_smem_doubles(int nk) {
-  return ((HC_PER_K * nk + 1) & ~1) + 13 * 32 + 20 * 32 + 2 * 2 * 33 + 2 * 2 * 66 + 64 + 3 * 32 * 32 + 8 +
+  return ((HC_PER_K * nk + 1) & ~1) + 13 * 32 + 20 * 32 + 2 * 2 * 33 + 2 * 2 * 66 + 64 + 3 * 32 * 32 + 8 + 1 +
          DUO_THREADS * (int)(sizeof(LaneCold) / 8) + (int)(sizeof(Cold) / 8);
 }
+static_assert((1 + DUO_THREADS * sizeof(LaneCold) / 8 + sizeof(Cold) / 8) % 2 == 0, "teams start 16-byte aligned");
 
-__device__ __forceinline__ DuoSmem duo_smem(double* p) {
+template <int TEAMS>
+__device__ __forceinline__ DuoSmem duo_smem(const DuoGeo<TEAMS>& g, double* p, int nk) {
   DuoSmem w;
-  w.up = p;
+  w.up = p + g.team * duo_smem_doubles(nk);
   w.ks = w.up + 13 * 32;
   w.xv = w.ks + 20 * 32;
   w.xr = w.xv + 2 * 2 * 33;
   w.rr = w.xr + 2 * 2 * 66;
   w.cm = w.rr + 64;
   w.red = w.cm + 3 * 32 * 32;
-  w.own = reinterpret_cast<LaneCold*>(w.red + 8);
+  w.claim = reinterpret_cast<int*>(w.red + 8);
+  w.own = reinterpret_cast<LaneCold*>(w.red + 9);
   w.cold = reinterpret_cast<Cold*>(w.own + DUO_THREADS);
   w.hc = reinterpret_cast<double*>(w.cold + 1);
-  if (threadIdx.x < 2) {
-    reinterpret_cast<double2*>(w.xv)[33 * threadIdx.x + 32] = make_double2(0.0, 0.0);
-    reinterpret_cast<double2*>(w.xr)[66 * threadIdx.x + 65] = make_double2(0.0, 0.0);
+  if (g.tid < 2) {
+    reinterpret_cast<double2*>(w.xv)[33 * g.tid + 32] = make_double2(0.0, 0.0);
+    reinterpret_cast<double2*>(w.xr)[66 * g.tid + 65] = make_double2(0.0, 0.0);
   }
-  if (threadIdx.x < 64) w.rr[threadIdx.x] = 0.0;
-  __syncthreads();
+  w.rr[g.tid] = 0.0;
+  duo_sync(g);
   return w;
 }
 
 // Constants of this thread's bubble (from its column of the caller's 13 rows)
 // and its coupling coefficients M(c, j, i) for the partners j = (i + d) mod K;
 // each lane of the pair writes half of them.  m points at M(0, 0, i).
-__device__ __forceinline__ void duo_store_bubble(const DuoSmem& W, const DuoGeo& g, const double* up13,
+template <int TEAMS>
+__device__ __forceinline__ void duo_store_bubble(const DuoSmem& W, const DuoGeo<TEAMS>& g, const double* up13,
                                                   long long up_stride, const MView& M) {
   if (g.valid)
     for (int p = g.c; p < 13; p += 2) W.up[p * 32 + g.i] = up13[p * up_stride];
@@ -104,8 +144,8 @@ __device__ __forceinline__ void duo_store_bubble(const DuoSmem& W, const DuoGeo&
 // d = 4 m + 2 c + e + 1; partners past K - 1 are the zero record with zero
 // coefficients, which adds nothing (straight-line code for 32 bubbles takes 46 us
 // an attempt, with a branch per four partners for K = 20 it took 75).
-template <int NKC, int ACC, bool FAST>
-__device__ __forceinline__ void duo_rhs_terms(const DuoGeo& g, const Params& P, const DuoSmem& W, const Cold& cold,
+template <int NKC, int ACC, bool FAST, int TEAMS>
+__device__ __forceinline__ void duo_rhs_terms(const DuoGeo<TEAMS>& g, const Params& P, const DuoSmem& W, const Cold& cold,
                                                double t, const double y[4], double D, double& b0, double& b1,
                                                double& cpf0, double (&Am)[16], double (&Bm)[16], double (&Cm)[16],
                                                double (&Dm)[16]) {
@@ -168,20 +208,22 @@ __device__ __forceinline__ void duo_rhs_terms(const DuoGeo& g, const Params& P, 
 }
 
 // Writes this thread's iterate and its bubble's squared residual to buffer
-// `buf` and waits for the block.  Two buffers used in turn need one barrier a
+// `buf` and waits for the team.  Two buffers used in turn need one barrier a
 // sweep.
-__device__ __forceinline__ void duo_exchange(const DuoGeo& g, const DuoSmem& W, int buf, double vr, double vt,
+template <int TEAMS>
+__device__ __forceinline__ void duo_exchange(const DuoGeo<TEAMS>& g, const DuoSmem& W, int buf, double vr, double vt,
                                               double rr) {
   if (g.valid) {
     reinterpret_cast<double2*>(W.xr)[66 * buf + g.i + (g.c ? g.K : 0)] = make_double2(vr, vt);
     if (g.c == 0) W.rr[32 * buf + g.i] = rr;
   }
-  __syncthreads();
+  duo_sync(g);
 }
 
 // Pairwise tree over the 32 (zero padded) squared residuals of buffer `buf`,
 // the same value in every thread.
-__device__ __forceinline__ double duo_norm(const DuoGeo& g, const DuoSmem& W, int buf) {
+template <int TEAMS>
+__device__ __forceinline__ double duo_norm(const DuoGeo<TEAMS>& g, const DuoSmem& W, int buf) {
   double v = W.rr[32 * buf + (g.tid & 31)];
 #pragma unroll
   for (int w = 1; w < 32; w <<= 1) v = v + __shfl_xor_sync(FULL, v, w);
@@ -190,7 +232,8 @@ __device__ __forceinline__ double duo_norm(const DuoGeo& g, const DuoSmem& W, in
 
 // Residual of the iterate in buffer `buf` (residual of the one-lane form): the
 // lane's two chains, joined with the other lane's.
-__device__ __forceinline__ void duo_residual(const DuoGeo& g, const DuoSmem& W, int buf, const double (&Am)[16],
+template <int TEAMS>
+__device__ __forceinline__ void duo_residual(const DuoGeo<TEAMS>& g, const DuoSmem& W, int buf, const double (&Am)[16],
                                               const double (&Bm)[16], const double (&Cm)[16], const double (&Dm)[16],
                                               double cpf0, double b0, double b1, double vr, double vt, double& r0,
                                               double& r1) {
@@ -215,7 +258,8 @@ __device__ __forceinline__ void duo_residual(const DuoGeo& g, const DuoSmem& W, 
   r1 = b1 - (st + vt);
 }
 
-__device__ __forceinline__ void duo_rhs(const DuoGeo& g, const Params& P, const DuoSmem& W, const Cold& cold,
+template <int TEAMS>
+__device__ __forceinline__ void duo_rhs(const DuoGeo<TEAMS>& g, const Params& P, const DuoSmem& W, const Cold& cold,
                                          double t, const double y[4], double dy[4], bool& conv, int& iters) {
   double2* xv2 = reinterpret_cast<double2*>(W.xv);
   if (g.valid) {
@@ -226,7 +270,7 @@ __device__ __forceinline__ void duo_rhs(const DuoGeo& g, const Params& P, const 
   const double D = fma(-(u7 * y[0]), y[2], y[0]) + W.up[4 * 32 + g.i] * u7;
   const bool general = g.valid & !(state_in_range(y[0], y[1], D) & (cold.normal != 0));
   double b0, b1, cpf0, Am[16], Bm[16], Cm[16], Dm[16];
-  if (__syncthreads_or(general))
+  if (duo_sync_or(g, general))
     duo_rhs_terms<0, -1, false>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);
   else if (P.nk == 2 && P.ac == 2)
     duo_rhs_terms<2, 2, true>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);
@@ -266,14 +310,15 @@ __device__ __forceinline__ void duo_rhs(const DuoGeo& g, const Params& P, const 
   dy[3] = vt;
 }
 
-// event_fun over the block (group_event of the one-lane form) and the step's
+// event_fun over the team (group_event of the one-lane form) and the step's
 // reductions: finiteness, acceptance, smallest ratio, event value.
-__device__ __forceinline__ double duo_event(const DuoGeo& g, const DuoSmem& W, const double y[4], double col,
+template <int TEAMS>
+__device__ __forceinline__ double duo_event(const DuoGeo<TEAMS>& g, const DuoSmem& W, const double y[4], double col,
                                              bool& fin, bool& ok, double& ratio) {
   double2* xv2 = reinterpret_cast<double2*>(W.xv);
   const double ri = y[0] * W.up[12 * 32 + g.i];
   if (g.valid && g.c == 0) xv2[g.i] = make_double2(ri, y[1]);
-  __syncthreads();
+  duo_sync(g);
   double gap = 1e30;
   if (g.i + 1 < g.K) {
     const double2 n = xv2[g.i + 1];
@@ -295,7 +340,7 @@ __device__ __forceinline__ double duo_event(const DuoGeo& g, const DuoSmem& W, c
     red[2] = bad_fin ? 1.0 : 0.0;
     red[3] = bad_ok ? 1.0 : 0.0;
   }
-  __syncthreads();
+  duo_sync(g);
   const double* a = W.red;
   gap = a[4] < a[0] ? a[4] : a[0];
   ratio = a[5] < a[1] ? a[5] : a[1];
@@ -304,9 +349,10 @@ __device__ __forceinline__ double duo_event(const DuoGeo& g, const DuoSmem& W, c
   return gap;
 }
 
-// One adaptive Cash-Karp step of the block's system.  Returns true if a dense
+// One adaptive Cash-Karp step of the team's system.  Returns true if a dense
 // sample must be stored after it.
-__device__ __forceinline__ bool duo_step(const DuoGeo& g, const Params& P, const DuoSmem& W, BubbleState& S) {
+template <int TEAMS>
+__device__ __forceinline__ bool duo_step(const DuoGeo<TEAMS>& g, const Params& P, const DuoSmem& W, BubbleState& S) {
   bool landing;
   double t_land;
   const double h = attempt_step(S, P, landing, t_land);

@@ -473,16 +473,15 @@ __global__ void __launch_bounds__(SOLO_THREADS, SOLO_BLOCKS)
 }
 
 // The same for 17 to 32 bubbles per system with the Richardson solve: one system
-// per block of two warps (duo_core.cuh).  KC: exact K, or 0 (read at run time).
-template <int KC>
-__global__ void __launch_bounds__(DUO_THREADS, DUO_BLOCKS)
+// per team of two warps (duo_core.cuh), TEAMS of them to a block, each claiming
+// for itself.  KC: exact K, or 0 (read at run time).
+template <int KC, int TEAMS>
+__global__ void __launch_bounds__(DUO_THREADS * TEAMS, DUO_BLOCKS / TEAMS)
     ensemble_duo_kernel(EnsLayout E, Params P, const int* __restrict__ order, int begin, int end, int K, int* head,
                          long long max_steps, int steps_total, const long long* epoch, long long budget_ns) {
   extern __shared__ __align__(16) double smem[];
-  __shared__ int claim;
-  __shared__ int over;
-  const DuoGeo g = make_duo_geo(KC > 0 ? KC : K);
-  const DuoSmem W = duo_smem(smem);
+  const DuoGeo<TEAMS> g = make_duo_geo<TEAMS>(KC > 0 ? KC : K);
+  const DuoSmem W = duo_smem(g, smem, P.nk);
   const long long deadline = budget_ns > 0 ? epoch[0] + budget_ns : 0;
   BubbleState S;
   S.c = W.cold;
@@ -496,10 +495,10 @@ __global__ void __launch_bounds__(DUO_THREADS, DUO_BLOCKS)
         const int n = begin + atomicAdd(head, 1);
         if (n < end) idx = order[n];
       }
-      claim = idx;
+      W.claim[0] = idx;
     }
-    __syncthreads();
-    const int sys = claim;
+    duo_sync(g);
+    const int sys = W.claim[0];
     if (sys < 0) break;
     const long long row = E.bubble_offset[sys] + (g.valid ? g.i : 0);
     if (g.tid == 0 && E.trace_load_ns) E.trace_load_ns[sys] = global_ns();
@@ -511,7 +510,7 @@ __global__ void __launch_bounds__(DUO_THREADS, DUO_BLOCKS)
     if (g.tid == 0)
       store_harmonics(W.hc, 1, sp[1], sp[2], sp[4], E.control_params + (long long)sys * E.cp_stride, P.nk, 1);
     ens_step_base(E, sys, steps_total, max_steps, S);
-    __syncthreads();
+    duo_sync(g);
     if (first_sample(S, P)) {
       if (g.valid && g.c == 0) ens_store_dense(E, S.t, S.y, S.c->boff, g.i, sys, S.o->idx);
       first_stored(S, P);
@@ -524,9 +523,9 @@ __global__ void __launch_bounds__(DUO_THREADS, DUO_BLOCKS)
     }
     while (S.active) {
       if (deadline != 0) {     // time slice over: stop after the current step
-        if (g.tid == 0) over = global_ns() >= deadline;
-        __syncthreads();
-        if (over) {
+        if (g.tid == 0) W.claim[1] = global_ns() >= deadline;
+        duo_sync(g);
+        if (W.claim[1]) {
           S.status = ST_MAX_STEPS;
           S.active = false;
           break;
@@ -584,7 +583,7 @@ cudaError_t launch_ensemble_k(const EnsLayout& E, const Params& P, const int* or
         kernel<<<blocks, threads, shmem, stream>>>(E, P, order, begin, end, head, max_steps, steps_total, epoch,
                                                    budget_ns, slots);
       } else if constexpr (KB == 32 && LIN == LIN_RICHARDSON) {
-        const auto kernel = ensemble_duo_kernel<KC>;
+        const auto kernel = threads == DUO_THREADS ? ensemble_duo_kernel<KC, 1> : ensemble_duo_kernel<KC, DUO_BLOCKS>;
         const cudaError_t e = configure_kernel(kernel, shmem);
         if (e != cudaSuccess) return e;
         kernel<<<blocks, threads, shmem, stream>>>(E, P, order, begin, end, K, head, max_steps, steps_total, epoch,
@@ -618,7 +617,7 @@ cudaError_t occupancy_k(int K, int nk, int threads, int lin, int mb, int* n) {
         configure_kernel(kernel, shmem);
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, threads, shmem);
       } else if constexpr (KB == 32 && LIN == LIN_RICHARDSON) {
-        const auto kernel = ensemble_duo_kernel<KC>;
+        const auto kernel = ensemble_duo_kernel<KC, 1>;
         configure_kernel(kernel, shmem);
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, threads, shmem);
       } else if constexpr (KB == 16 && LIN == LIN_RICHARDSON) {

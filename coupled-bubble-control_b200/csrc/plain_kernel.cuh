@@ -244,8 +244,8 @@ template <int KC>
 __global__ void __launch_bounds__(DUO_THREADS, DUO_BLOCKS)
     plain_duo_kernel(RefLayout L, Params P, long long budget, int final_launch, int* active_counter) {
   extern __shared__ __align__(16) double smem[];
-  const DuoGeo g = make_duo_geo(KC > 0 ? KC : L.ups);
-  const DuoSmem W = duo_smem(smem);
+  const DuoGeo<1> g = make_duo_geo<1>(KC > 0 ? KC : L.ups);
+  const DuoSmem W = duo_smem(g, smem, P.nk);
   const long long s = blockIdx.x;
   const long long NST = (long long)L.ns * L.tile;
   const long long lane_off = s * L.tile + (g.valid ? g.i : 0);

@@ -1,12 +1,12 @@
-"""Time slices, resumed solves, step caps, traces and sparse warps for every
-kernel form (one system per lane, one lane per bubble, padded
+"""Time slices, resumed solves, step caps, traces, sparse warps and latency
+lanes for every kernel form (one system per lane, one lane per bubble, padded
 and exact, two lanes per bubble), in one batch with backfill grids.  Every
 output equals that of one uninterrupted solve bit for bit."""
 import numpy as np
 import pytest
 
 from cbc_b200 import scenes
-from cbc_b200.ensemble import Ensemble, make_work_list
+from cbc_b200.ensemble import Ensemble, WorkList, make_work_list
 
 pytestmark = pytest.mark.gpu
 
@@ -73,5 +73,30 @@ def test_sparse_warps_equal_one_solve(single, slots):
     wl = make_work_list(e.host["K"], e.host["t_end"])
     wl.slots = np.asarray([1 if slots == "one" else max(1, 16 // int(k)) for k in wl.bucket_K], np.int32)
     e.solve(100_000, work=wl)
+    torch.cuda.synchronize()
+    compare(e.to_host(), single[100_000])
+
+
+@pytest.mark.parametrize("budget_ns", [0, 400_000])
+def test_latency_lanes_of_every_form_equal_one_solve(single, budget_ns):
+    """Two exclusive SMs per bubble count, the rest in ordinary buckets."""
+    import torch
+    e = batch()
+    K = e.host["K"]
+    order, bk, ex = [], [], []
+    for k in sorted(BATCH):
+        ids = np.nonzero(K == k)[0].astype(np.int32)
+        n = max(5, ids.size // 3)
+        order += [ids[:n], ids[n:]]
+        bk += [k, k]
+        ex += [2, 0]
+    wl = WorkList(order=np.concatenate(order), bucket_K=np.asarray(bk, np.int32),
+                  bucket_begin=np.concatenate([[0], np.cumsum([o.size for o in order])]).astype(np.int32),
+                  exclusive=np.asarray(ex, np.int32))
+    for _ in range(2000):
+        e.solve(100_000, work=wl, budget_ns=budget_ns, steps_total=True)
+        st = e.dev["status"].cpu().numpy()
+        if not np.any((st == 0) | (st == -1)):
+            break
     torch.cuda.synchronize()
     compare(e.to_host(), single[100_000])
