@@ -13,7 +13,7 @@
 //     measured).  rcp() and quot() below have none.
 //   * Rounding to an integer, conversion to int and scaling by 2^n are an
 //     addition of 1.5 2^52 and integer operations on the exponent field.
-// The caller guarantees the ranges given at each function (system_in_range and
+// The caller guarantees the ranges given at each function (fast_until and
 // state_in_range test them; outside, the general functions are taken).
 #pragma once
 

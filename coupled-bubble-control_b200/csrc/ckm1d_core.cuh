@@ -160,7 +160,7 @@ __device__ __forceinline__ double tree_open(double (&a)[N], int n) {
 
 // Per-warp shared-memory carve-up, in doubles.
 struct WarpSmem {
-  double* hc;   // [7 nk][G]   harmonic constants of each group (component-major)
+  double* hc;   // [7 nk + 1][G] harmonic constants of each group (component-major); fast_until
   double* up;   // [15][32]    bubble constants, lane-private columns
   double* ks;   // [6][4][32]  stage derivatives, lane-private columns
   double* xv;   // [2][32] double2 partner-state exchange records
@@ -176,7 +176,7 @@ enum : int { LIN_RICHARDSON = 0, LIN_LU = 1 };
 
 // Harmonic-constant region rounded up to an even count, so that every later
 // region (and every warp's carve-up) stays 16-byte aligned for double2 access.
-__host__ __device__ inline int hc_doubles(int K, int nk) { return (HC_PER_K * nk * (32 / K) + 1) & ~1; }
+__host__ __device__ inline int hc_doubles(int K, int nk) { return ((HC_PER_K * nk + 1) * (32 / K) + 1) & ~1; }
 
 // Matrix region per warp (direct solve only):
 //   K <= 8: staging of the four coefficient blocks by absolute column,
@@ -238,7 +238,6 @@ struct LaneState {
   int idx;                     // dense samples stored
   int status;
   bool active;
-  bool normal;                 // constants and phases within the range of the fast functions
   int steps, rejected, conv_ok, conv_fail;
   long long lin_iters;
 };
@@ -283,6 +282,10 @@ __device__ __forceinline__ void store_harmonics(double* hc, int stride, double s
 
 __device__ __forceinline__ double hcv(const WarpSmem& w, const Geo& g, int k, int c) {
   return w.hc[(HC_PER_K * k + c) * g.G + g.grp];
+}
+
+__device__ __forceinline__ double& fast_until_of(const WarpSmem& w, const Geo& g, int nk) {
+  return w.hc[HC_PER_K * nk * g.G + g.grp];
 }
 
 // Pairwise-tree sum of v over the group (next power of two, zero padded):
@@ -635,20 +638,25 @@ __device__ __forceinline__ void f_sincos(double x, double* s, double* c) {
   }
 }
 
-// Range of the FAST forms.  Constants and phases of a system, tested once when
-// it is loaded (sp0, sp1, sp2: system parameters; cp[m cp_stride]: control
-// parameters as in store_harmonics): 3 gamma <= 15, phases below 2^50 up to
-// t_end and for positions below 2^32.
-__device__ __forceinline__ int system_in_range(double sp0, double sp1, double sp2, const double* cp, int nk,
-                                               long long cp_stride, double t, double t_end) {
-  const double tm = fabs(t) > fabs(t_end) ? fabs(t) : fabs(t_end);
-  bool ok = fabs(sp0) <= 15.0;
+// Range of the FAST forms.  Largest |t| up to which the phases of a system in time
+// are below 2^50, found once when it is loaded; negative if its constants put it
+// outside at any time (sp0, sp1, sp2: system parameters; cp[m cp_stride]: control
+// parameters as in store_harmonics): 3 gamma <= 15, phases in space below 2^50 for
+// positions below 2^32.  The phases are tested at the times of an attempt and not
+// at t_end, which may be far beyond any time that is reached.  t: the time when it
+// is loaded; no later time is smaller, so an attempt has to test its end alone.
+__device__ __forceinline__ double fast_until(double sp0, double sp1, double sp2, const double* cp, int nk,
+                                             long long cp_stride, double t) {
+  double until = fabs(sp0) <= 15.0 ? 0x1p1000 : -1.0;
   for (int k = 0; k < nk; ++k) {
     const double omega = cp[(nk + k) * cp_stride], phase = cp[(2 * nk + k) * cp_stride],
                  wave = cp[(3 * nk + k) * cp_stride];
-    ok = ok && fma(fabs(TWO_PI * sp1 * omega), tm, fabs(phase)) < 0x1p50 && fabs(TWO_PI * sp2 * wave) < 0x1p17;
+    const double room = 0x1p50 - fabs(phase), w = fabs(TWO_PI * sp1 * omega);
+    const bool ok = (room > 0.0) & (fabs(TWO_PI * sp2 * wave) < 0x1p17) & (w < 0x1p500);
+    const double u = room / w;          // infinite for a constant phase
+    until = ok ? (u < until ? u : until) : -1.0;
   }
-  return ok ? 1 : 0;
+  return fabs(t) <= until ? until : -1.0;
 }
 // Arguments of one evaluation: radius (dimensionless) in [2^-64, 2^64), so
 // that |3 gamma log R| < 690; position below 2^32 (so pair distances are at
@@ -1076,10 +1084,22 @@ __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSm
   // compiled right-hand side: two harmonics of a standing wave with the antinode
   // (SW_A) or the node (SW_N) at x = 0, the forms of the benchmarked workloads;
   // any other form uses the general one (P is uniform over a launch, so the
-  // branch never diverges), and so does an attempt in which some argument of the
-  // warp was outside the range of the fast functions: it is evaluated again.
-  constexpr bool FAST = LIN == LIN_RICHARDSON;
+  // branch never diverges), and so does a warp that holds a system outside the
+  // range of the fast functions.  An attempt in which some state of the warp
+  // left that range is evaluated again.
+  // The form is held in two flags, for two bubbles in one and P.ac (no register is
+  // left): an attempt alone in one flag / two, K = 2 10.2 us / 10.8 (16 bytes
+  // spilled), 3 13.4 / 12.6, 5 22.0 / 18.3, 6 22.9 / 18.4, 4, 7 and 8 the same.
+  constexpr bool FAST = LIN == LIN_RICHARDSON, FLAGS = FAST && KB > 2;
   bool general = P.nk != 2 || P.ac == 0;
+  if constexpr (FAST) {
+    // (fabs(t) + h orders the code otherwise: GPU full 0.660 ns an attempt against
+    // 0.622 with t + h for two bubbles, 1.372 against 1.390 for three)
+    const double reached = FLAGS ? fabs(t) + h : t + h;
+    const bool outside = __any_sync(FULL, on & !(reached <= fast_until_of(W, g, P.nk)));
+    general = general | outside;
+  }
+  bool swa = !general & (P.ac == 2), swn = !general & (P.ac == 1);
   int conv_fail_here, sweeps;
   while (true) {
     bool in_range = true;
@@ -1102,9 +1122,9 @@ __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSm
       double kk[4];
       bool cv, ok;
       int it;
-      if (!general && P.ac == 2)
+      if (FLAGS ? swa : !general && P.ac == 2)
         rhs_form<KB, KC, LIN, 2, 2, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
-      else if (!general)
+      else if (FLAGS ? swn : !general)
         rhs_form<KB, KC, LIN, 2, 1, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
       else
         rhs_form<KB, KC, LIN, 0, -1, false>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
@@ -1114,9 +1134,10 @@ __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSm
       sweeps += it;
       conv_fail_here += cv ? 0 : 1;
     }
-    if (!FAST || general) break;
-    if (__all_sync(FULL, !on | (in_range & S.normal))) break;
+    if (!FAST || (FLAGS ? !(swa | swn) : general)) break;
+    if (__all_sync(FULL, !on | in_range)) break;
     general = true;
+    swa = swn = false;
   }
   if (on) {
     S.lin_iters += sweeps;

@@ -18,12 +18,11 @@ struct Cold {
   double t_end, t_begin;
   double ddt;                  // spacing of the dense samples
   long long boff, step_base;   // batched form: first bubble row; steps accumulated before this load
-  int normal;                  // constants and phases within the range of the interleaved functions
+  double fast_until;           // range of the interleaved functions
   int rejected, conv_ok, conv_fail;
   long long lin_iters;
-  long long pad;               // odd multiple of 8 bytes: neighbouring records on different banks
 };
-static_assert(sizeof(Cold) % 16 == 8, "odd multiple of 8 bytes");
+static_assert(sizeof(Cold) % 16 == 8, "odd multiple of 8 bytes: neighbouring records on different banks");
 // The ones that every lane of a system updates for itself.
 struct LaneCold {
   double dnext;                // next dense sample time

@@ -268,7 +268,7 @@ __device__ __forceinline__ void duo_rhs(const DuoGeo<TEAMS>& g, const Params& P,
   }
   const double u7 = W.up[7 * 32 + g.i];
   const double D = fma(-(u7 * y[0]), y[2], y[0]) + W.up[4 * 32 + g.i] * u7;
-  const bool general = g.valid & !(state_in_range(y[0], y[1], D) & (cold.normal != 0));
+  const bool general = g.valid & !(state_in_range(y[0], y[1], D) & (fabs(t) <= cold.fast_until));
   double b0, b1, cpf0, Am[16], Bm[16], Cm[16], Dm[16];
   if (duo_sync_or(g, general))
     duo_rhs_terms<0, -1, false>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);

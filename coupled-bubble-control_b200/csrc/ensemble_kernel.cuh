@@ -67,8 +67,7 @@ __device__ __forceinline__ void ens_load_scalars(const EnsLayout& E, const Param
     S.c->sp0 = sp[0];
     S.c->sp3 = sp[3];
     S.c->boff = E.bubble_offset[s];
-    S.c->normal = system_in_range(sp[0], sp[1], sp[2], E.control_params + (long long)s * E.cp_stride, P.nk, 1, S.t,
-                                  t_end);
+    S.c->fast_until = fast_until(sp[0], sp[1], sp[2], E.control_params + (long long)s * E.cp_stride, P.nk, 1, S.t);
   }
   prologue(S, P, t_end, E.t_begin[s], E.event[s], ens_prev_time(E, P, s, S.o->idx), E.status[s]);
 }
@@ -112,6 +111,7 @@ __device__ __forceinline__ void ens_write_scalars(const EnsLayout& E, const Para
 
 // Loads system s into this lane's slot (lane li of the group) and runs the
 // prologue.  Called only by lanes whose group claimed s.
+template <int LIN>
 __device__ __forceinline__ void lane_load(const EnsLayout& E, const Params& P, const Geo& g, int s, LaneState& S,
                                          const WarpSmem& W, long long& boff) {
   boff = E.bubble_offset[s];
@@ -127,11 +127,14 @@ __device__ __forceinline__ void lane_load(const EnsLayout& E, const Params& P, c
   S.t_begin = E.t_begin[s];
   S.h = E.h[s];
   S.idx = (P.ndo > 0) ? E.dense_index[s] : 0;
-  S.normal = system_in_range(sp[0], sp[1], sp[2], E.control_params + (long long)s * E.cp_stride, P.nk, 1, S.t,
-                             S.t_end) != 0;
   prologue(S, P, E.event[s], ens_prev_time(E, P, s, S.idx), E.status[s]);
   store_coupling(W, g, MView{E.coupling + E.coupling_offset[s] + g.li, (long long)g.K * g.K, g.K});
-  if (g.li == 0) store_harmonics(W.hc + g.grp, g.G, sp[1], sp[2], sp[4], E.control_params + (long long)s * E.cp_stride, P.nk, 1);
+  if (g.li == 0) {
+    const double* cp = E.control_params + (long long)s * E.cp_stride;
+    store_harmonics(W.hc + g.grp, g.G, sp[1], sp[2], sp[4], cp, P.nk, 1);
+    if constexpr (LIN == LIN_RICHARDSON)
+      fast_until_of(W, g, P.nk) = fast_until(sp[0], sp[1], sp[2], cp, P.nk, 1, S.t);
+  }
 }
 
 __device__ __forceinline__ void lane_writeback(const EnsLayout& E, const Params& P, const Geo& g, int s,
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(128, min_blocks_variant(KB, MB))
       const bool fresh = g.valid && sys < 0 && got >= 0 && leader_wanted != 0;
       if (fresh) {
         sys = got;
-        lane_load(E, P, g, sys, S, W, boff);
+        lane_load<LIN>(E, P, g, sys, S, W, boff);
         step_base = (steps_total && E.steps) ? (long long)E.steps[sys] : 0;
         if (S.active && step_base >= max_steps) {
           S.status = ST_MAX_STEPS;

@@ -37,9 +37,9 @@ __device__ __forceinline__ double ref_prev_time(const RefLayout& L, const Params
   return (P.ndo > 0 && idx > 0) ? L.dense_time[(long long)(idx - 1) * L.ns + s] : 0.0;
 }
 
-__device__ __forceinline__ int ref_in_range(const RefLayout& L, const Params& P, long long s, double t, double t_end) {
-  return system_in_range(L.system_params[0 * (long long)L.ns + s], L.system_params[1 * (long long)L.ns + s],
-                         L.system_params[2 * (long long)L.ns + s], L.control_params + s, P.nk, L.ns, t, t_end);
+__device__ __forceinline__ double ref_fast_until(const RefLayout& L, const Params& P, long long s, double t) {
+  return fast_until(L.system_params[0 * (long long)L.ns + s], L.system_params[1 * (long long)L.ns + s],
+                    L.system_params[2 * (long long)L.ns + s], L.control_params + s, P.nk, L.ns, t);
 }
 
 // Scalars of system s into a lane's state, and the prologue: scalars in
@@ -52,7 +52,6 @@ __device__ __forceinline__ void ref_load(const RefLayout& L, const Params& P, lo
   S.t_begin = L.time_begin[s];
   S.h = L.time_step[s];
   S.idx = (P.ndo > 0) ? L.dense_index[s] : 0;
-  S.normal = ref_in_range(L, P, s, S.t, S.t_end) != 0;
   prologue(S, P, L.actual_event[s], ref_prev_time(L, P, s, S.idx), L.status[s]);
 }
 __device__ __forceinline__ void ref_load(const RefLayout& L, const Params& P, long long s, ScalarState& S) {
@@ -63,7 +62,7 @@ __device__ __forceinline__ void ref_load(const RefLayout& L, const Params& P, lo
   if (S.lead) {
     S.c->sp0 = L.system_params[0 * (long long)L.ns + s];
     S.c->sp3 = L.system_params[3 * (long long)L.ns + s];
-    S.c->normal = ref_in_range(L, P, s, S.t, t_end);
+    S.c->fast_until = ref_fast_until(L, P, s, S.t);
   }
   prologue(S, P, t_end, L.time_begin[s], L.actual_event[s], ref_prev_time(L, P, s, S.o->idx), L.status[s]);
 }
@@ -123,7 +122,10 @@ __global__ void __launch_bounds__(128, min_blocks_for(KB))
     store_bubble_consts(W, g, L.unit_params + lane_off, NST);
     store_coupling(W, g, MView{L.coupling + lane_off, (long long)L.ups * NST, NST});
     ref_load(L, P, s, S);
-    if (g.li == 0) ref_store_harmonics(L, P, s, W.hc + g.grp, g.G);
+    if (g.li == 0) {
+      ref_store_harmonics(L, P, s, W.hc + g.grp, g.G);
+      if constexpr (LIN == LIN_RICHARDSON) fast_until_of(W, g, P.nk) = ref_fast_until(L, P, s, S.t);
+    }
   }
   __syncwarp();
   if (have && first_sample(S, P)) {

@@ -58,7 +58,7 @@ __device__ __forceinline__ void solo_rhs_form(const Params& P, const SoloSmem& W
   const auto up = [&](int p) { return W.up[p * 32 + lane]; };
   const double u7 = up(7);
   const double D = fma(-(u7 * y[0]), y[2], y[0]) + up(4) * u7;
-  in_range = (cold.normal != 0) & state_in_range(y[0], y[1], D);
+  in_range = state_in_range(y[0], y[1], D);
   const OwnTerms o = own_terms<NKC, ACC, FAST, false>(P, hc, cold.sp0, t, y[0], y[1], D, 0, 0);
   double b0, b1;
   implicit_rhs(o, PairSums{0.0, 0.0, 0.0, 0.0, 0.0}, up, cold.sp3, y[0], y[2], y[3], b0, b1);
@@ -93,9 +93,10 @@ __device__ __forceinline__ bool solo_step(const Params& P, const SoloSmem& W, in
   double* ks = W.ks + lane;     // ks[(st * 4 + c) * 32]
   int conv_fail_here, sweeps;
   double kk[4];
-  // the attempt is made again with the general functions when an argument of
-  // some lane was outside the range of the interleaved ones
-  for (bool general = false;; general = true) {
+  // the general functions where some lane's system is outside the range of the
+  // interleaved ones; made again with them when some lane's state left it
+  const bool outside = __any_sync(FULL, on & !(S.t + h <= S.c->fast_until));
+  for (bool general = outside;; general = true) {
     bool in_range = true;
     conv_fail_here = sweeps = 0;
 #pragma unroll 1

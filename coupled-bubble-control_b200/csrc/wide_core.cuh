@@ -180,17 +180,17 @@ __device__ __forceinline__ void wide_rhs(const Geo& g, const Params& P, const Wi
   __syncwarp();
   const double u7 = upv(W, g, 7);
   const double D = fma(-(u7 * y[0]), y[2], y[0]) + upv(W, g, 4) * u7;
-  const bool general = on & !(state_in_range(y[0], y[1], D) & (cold.normal != 0));
+  const bool general = on & !(state_in_range(y[0], y[1], D) & (fabs(t) <= cold.fast_until));
   double b0, b1, cpf0, Am[WIDE], Bm[WIDE], Cm[WIDE], Dm[WIDE];
-  if (P.nk == 2 && P.ac == 2)
+  // some lane's arguments are outside the range of the interleaved functions
+  if (__any_sync(FULL, general))
+    wide_rhs_terms<0, -1, false>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);
+  else if (P.nk == 2 && P.ac == 2)
     wide_rhs_terms<2, 2, true>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);
   else if (P.nk == 2 && P.ac == 1)
     wide_rhs_terms<2, 1, true>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);
   else
     wide_rhs_terms<0, -1, true>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);
-  // an argument of some lane was outside the range of the interleaved functions
-  if (__any_sync(FULL, general))
-    wide_rhs_terms<0, -1, false>(g, P, W, cold, t, y, D, b0, b1, cpf0, Am, Bm, Cm, Dm);
 
   // relaxed Richardson from v = b, two sweeps per vote (see rhs_form in
   // ckm1d_core.cuh)
