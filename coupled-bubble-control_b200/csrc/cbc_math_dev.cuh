@@ -25,25 +25,46 @@ namespace cbcd {
 // rint), and leaves that integer's two's complement in the low word.
 constexpr double RINT_MAGIC = 6755399441055744.0;
 
-// 1/x correctly rounded, for 2^-1000 <= |x| <= 2^1000.
-// Seed with relative error e0 < 2^-19.9 (measured), third-order step
-// y = y0 (1 + e0 + e0^2) with error e0^3 < 2^-59 before its rounding, then
-// Markstein's correction y + y (1 - x y) (P. Markstein, "IA-64 and Elementary
-// Functions", 2000, ch. 8): 1 - x y is exact, the corrected value differs from
-// 1/x by e^2 / x with |e| the relative error of the rounded y.  A 53-bit
-// quotient 1/x misses a rounding boundary by 2^-106 at least, and only where
-// the significand X of x divides 2^106 - 1 with a 53-bit X: the only divisor
-// of (2^53 - 1)(2^53 + 1) in [2^52, 2^53) is 2^53 - 1.  For that X the
-// correction ends on the lower neighbour, so rcp_last adds one unit.
-__device__ __forceinline__ double rcp_last(double x, double y) {
-  const unsigned ones = (unsigned)__double2loint(x) & ((unsigned)__double2hiint(x) | 0xfff00000u);
-  return __hiloint2double(__double2hiint(y), __double2loint(y) + (ones == 0xffffffffu ? 1 : 0));
+// 1/x correctly rounded, for 2^-1000 <= |x| <= 2^1000, from a seed y of relative
+// error |e0| < 2^-19, e0 = 1 - x y.  Three terms of the geometric series
+// 1/x = y / (1 - e0) = y (1 + e0 + e0^2 + ...) leave e0^3 < 2^-57 before their
+// rounding, then Markstein's correction y + y (1 - x y) (P. Markstein, "IA-64 and
+// Elementary Functions", 2000, ch. 8): 1 - x y is exact, the corrected value differs
+// from 1/x by e^2 / x with |e| the relative error of the rounded y.  A 53-bit
+// quotient 1/x misses a rounding boundary by 2^-106 at least, and only where the
+// significand X of x divides 2^106 - 1 with a 53-bit X: the only divisor of
+// (2^53 - 1)(2^53 + 1) in [2^52, 2^53) is 2^53 - 1.  There 1/x lies just above the
+// middle of 2^-k and its upper neighbour, which it rounds to; the correction ends
+// on either of the two, with the sign of the seed's error, and both have the same
+// high word, so the low word is set.
+CBC_HD int low_word(double x) {
+#if defined(__CUDA_ARCH__)
+  return __double2loint(x);
+#else
+  return (int)(uint32_t)cbcm::double_to_bits(x);
+#endif
+}
+CBC_HD int high_word(double x) {
+#if defined(__CUDA_ARCH__)
+  return __double2hiint(x);
+#else
+  return (int)(uint32_t)(cbcm::double_to_bits(x) >> 32);
+#endif
+}
+CBC_HD double join_words(int hi, int lo) {
+#if defined(__CUDA_ARCH__)
+  return __hiloint2double(hi, lo);
+#else
+  return cbcm::bits_to_double((uint64_t)(uint32_t)hi << 32 | (uint32_t)lo);
+#endif
+}
+CBC_HD double rcp_last(double x, double y) {
+  const unsigned ones = (unsigned)low_word(x) & ((unsigned)high_word(x) | 0xfff00000u);
+  return join_words(high_word(y), ones == 0xffffffffu ? 1 : low_word(y));
 }
 template <int N>
-__device__ __forceinline__ void rcp(const double (&x)[N], double (&y)[N]) {
+CBC_HD void rcp_refine(const double (&x)[N], double (&y)[N]) {
   double e[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y[i]) : "d"(x[i]));
 #pragma unroll
   for (int i = 0; i < N; ++i) e[i] = fma(-x[i], y[i], 1.0);
 #pragma unroll
@@ -54,6 +75,14 @@ __device__ __forceinline__ void rcp(const double (&x)[N], double (&y)[N]) {
   for (int i = 0; i < N; ++i) e[i] = fma(-x[i], y[i], 1.0);
 #pragma unroll
   for (int i = 0; i < N; ++i) y[i] = rcp_last(x[i], fma(e[i], y[i], y[i]));
+}
+// The seed: relative error 2^-19.9 at most over all high words of the significand
+// (measured), the only part of x that it depends on.
+template <int N>
+__device__ __forceinline__ void rcp(const double (&x)[N], double (&y)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y[i]) : "d"(x[i]));
+  rcp_refine(x, y);
 }
 
 // a/b correctly rounded, for a and b with exponents well inside the range (no
