@@ -22,7 +22,9 @@ using namespace cbc;
 
 extern "C" {
 
-int32_t cbc_version(void) { return 100; }
+// Raised with every change of the kernels: launch shapes tuned on one version are
+// not used by another (the tuner's table has it in its keys).
+int32_t cbc_version(void) { return 101; }
 
 int32_t cbc_create(cbc_context** out, int32_t device) {
   if (!out) return fail(nullptr, CBC_E_INVALID, "out is NULL");
