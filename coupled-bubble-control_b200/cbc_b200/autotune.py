@@ -7,8 +7,8 @@ become compile-time macros, and the register cap is a build option
 ``max_registers`` in ``backends/cuda_opts.py:6-73``).  Here the kernels are
 prebuilt for sm_100a and the shape is chosen at run time by measurement:
 
-* ``threads``     threads per block (32 .. 128; K = 32 is cut further to the
-                  warps whose shared memory fits);
+* ``threads``     threads per block (32 .. 128; the direct solve at K = 32 is cut
+                  further to the warps whose shared memory fits);
 * ``slots``       systems a warp holds (32 // K, or half of it: idle lanes
                   for less intra-warp divergence of the Richardson iteration);
 * ``min_blocks``  the register-budget variant of the kernel (0: the
@@ -21,9 +21,9 @@ current step when the slice ends, cbc_work.budget_ns), from the same
 initial state, and keeps the candidate with the most step attempts per
 second.  Results never depend on the shape (per-system arithmetic is the
 same in every lane arrangement), so tuning is free to change between runs.
-The table is cached per device name, library version, harmonics count and
-linear solver in a JSON file (``$CBC_TUNE_CACHE`` or
-``~/.cache/cbc_b200/autotune.json``).
+The table is cached per device name, library version (raised with every change
+of the kernels), harmonics count and linear solver in a JSON file
+(``$CBC_TUNE_CACHE`` or ``~/.cache/cbc_b200/autotune.json``).
 """
 from __future__ import annotations
 
@@ -61,6 +61,18 @@ def candidates(K: int) -> List[TuneConfig]:
             for mb in mb_opts:
                 out.append(TuneConfig(th, sl, mb))
     return out
+
+
+def launch_shape(K: int, cfg: TuneConfig, lin_solver: str) -> tuple:
+    """What the kernel of K bubbles and this solver takes from `cfg`: the
+    Richardson kernels of a single bubble have one register budget, those of more
+    than 16 a fixed block of two warps per system."""
+    threads, slots, mb = cfg.threads, cfg.slots, cfg.min_blocks
+    if lin_solver == "richardson" and K == 1:
+        mb = 0
+    if lin_solver == "richardson" and K > 16:
+        threads = 64
+    return threads, slots, mb
 
 
 def choose(rates: Dict[TuneConfig, float], margin: float = 0.02) -> TuneConfig:
@@ -107,10 +119,17 @@ def save_cache(table: Dict[str, dict], path: Optional[str] = None) -> None:
         pass   # a read-only home only costs a re-tune next time
 
 
-def tune_k(K: int, measure: Callable[[TuneConfig], float], repeats: int = 2) -> Dict:
-    """Measures every candidate for K (best of `repeats`) and picks one."""
+def tune_k(K: int, measure: Callable[[TuneConfig], float], repeats: int = 2, lin_solver: str = "richardson") -> Dict:
+    """Measures every candidate for K (best of `repeats`) and picks one.  Of
+    candidates that launch the same kernel the same way only the first is
+    measured, so that noise does not choose between them."""
     rates: Dict[TuneConfig, float] = {}
+    seen = set()
     for cfg in candidates(K):
+        shape = launch_shape(int(K), cfg, lin_solver)
+        if shape in seen:
+            continue
+        seen.add(shape)
         rates[cfg] = max(measure(cfg) for _ in range(repeats))
     best = choose(rates)
     return {"config": best, "rates": {c.label(): r for c, r in rates.items()},
@@ -178,7 +197,7 @@ class Autotuner:
                 out[K] = TuneConfig(**hit["config"])
                 self.report[K] = dict(hit, cached=True)
                 continue
-            res = tune_k(K, self._pilot(ens, K))
+            res = tune_k(K, self._pilot(ens, K), lin_solver=lin)
             out[K] = res["config"]
             entry = {"config": asdict(res["config"]), "rates": res["rates"],
                      "gain_vs_default": res["gain_vs_default"]}
