@@ -682,8 +682,9 @@ def run_b200(args):
 
 def cost_tables(dev_index: int = 0, seconds: float = 0.5):
     """Per-K cost tables of the adaptive scheduler: the steady cost of one
-    step attempt with the GPU full (ns: the K bucket of the mixed-K workload,
-    a device-time slice of `seconds` from t = 0), the latency of one attempt
+    step attempt with the GPU full (ns: the K bucket of the mixed-K workload, or
+    systems of the same kind where it has none of that K, a device-time slice of
+    `seconds` from t = 0), the latency of one attempt
     of a system alone (us) and, from the same slice, the latency one attempt
     sees inside the full GPU (us, 90th percentile of the systems' attempt
     counts) over the alone latency (the load factor)."""
@@ -692,10 +693,15 @@ def cost_tables(dev_index: int = 0, seconds: float = 0.5):
     from cbc_b200.ensemble import Ensemble
     torch.cuda.set_device(dev_index)
     mix = scenes.mixed_k(ns=65536, seed=1)
-    one = scenes.uniform(1, ns=26214, periods=20.0, seed=91)
     step_ns, alone_us, bulk_us = {}, {}, {}
-    for k in (1, 2, 3, 4, 6, 8):
-        sc = one if k == 1 else scenes.subset(mix, np.nonzero(mix.K == k)[0])
+    for k in (1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 15, 16, 17, 31, 32):
+        if np.any(mix.K == k):
+            sc = scenes.subset(mix, np.nonzero(mix.K == k)[0])
+        else:
+            # several rounds of the systems that fill the GPU
+            ns = 160000 if k == 1 else (16000 if k <= 8 else (10000 if k <= 16 else 2500))
+            sc = scenes.uniform(k, ns=ns, periods=20.0, seed=90 + k, pa_hi=1.5 if k <= 8 else 1.2,
+                                x_range=(-0.25, 0.25) if k <= 8 else (-0.5, 0.5))
         ens = Ensemble.from_scene(sc, device=dev_index).to_device()
         ens.solve(200)
         ens.reset_device()
@@ -709,7 +715,7 @@ def cost_tables(dev_index: int = 0, seconds: float = 0.5):
         att = (ens.dev["steps"] + ens.dev["rejected"]).cpu().numpy().astype(np.float64)
         step_ns[k] = ms * 1e6 / float(att.sum())
         bulk_us[k] = ms * 1e3 / float(np.percentile(att, 90))
-        alone_us[k] = alone_latency(sc if k == 1 else mix, dev_index, "richardson", ks=(k,))[f"K{k}_us_per_attempt"]
+        alone_us[k] = alone_latency(sc, dev_index, "richardson", ks=(k,))[f"K{k}_us_per_attempt"]
     return {"workload": "cost_tables", "slice_s": seconds, "step_ns": step_ns, "alone_us": alone_us,
             "bulk_us": bulk_us, "load_factor": {k: bulk_us[k] / alone_us[k] for k in step_ns}}
 

@@ -40,35 +40,32 @@ class WorkList:
 
 
 # Steady-state cost of one step attempt on a full B200 (ns), measured on the
-# K buckets of the mixed-K workload filling the GPU (a 0.5 s slice from t = 0;
-# `python bench.py --workload costs`); other K are interpolated.
-STEP_NS = {1: 0.58, 2: 0.846, 3: 2.14, 4: 2.55, 6: 6.32, 8: 7.16}
+# K buckets of the mixed-K workload and on systems of the same kind for the K it
+# has none of (a 0.5 s slice from t = 0; `python bench.py --workload costs`).  The
+# ends of every kernel form are measured; inside a form (9..15 are padded to 16,
+# 17..31 to 32) the cost is nearly the same and interpolated.
+STEP_NS = {1: 0.148, 2: 0.817, 3: 1.83, 4: 2.48, 5: 3.71, 6: 5.47, 7: 6.29, 8: 6.33, 9: 21.9, 10: 22.4, 11: 33.4,
+           15: 36.3, 16: 23.7, 17: 118.0, 31: 128.0, 32: 113.0}
 # Latency of one step attempt of a system whose warp has an SM sub-partition
-# to itself (us), measured on single systems of the mixed-K workload.
-ALONE_US = {1: 9.3, 2: 13.9, 3: 15.8, 4: 14.8, 6: 23.5, 8: 23.9}
+# to itself (us), measured on single systems of the same workloads.
+ALONE_US = {1: 5.17, 2: 11.8, 3: 11.9, 4: 14.0, 5: 17.2, 6: 18.5, 7: 19.1, 8: 19.4, 9: 55.3, 10: 55.5, 11: 55.5,
+            15: 55.9, 16: 39.0, 17: 56.8, 31: 55.6, 32: 48.4}
+
+
+def _per_bubble_count(table: Dict[int, float], K) -> np.ndarray:
+    ks = sorted(table)
+    return np.interp(np.atleast_1d(np.asarray(K, dtype=np.float64)), ks, [table[k] for k in ks])
 
 
 def cost_weight(K) -> np.ndarray:
     """Relative cost of one step of a K-bubble system (ns on a full GPU)."""
-    K = np.atleast_1d(np.asarray(K, dtype=np.float64))
-    ks = np.asarray(sorted(STEP_NS), dtype=np.float64)
-    vs = np.asarray([STEP_NS[int(k)] for k in ks])
-    out = np.interp(K, ks, vs)
-    big = K > ks[-1]
-    out[big] = vs[-1] * (K[big] / ks[-1]) ** 2
-    return out
+    return _per_bubble_count(STEP_NS, K)
 
 
 def alone_latency(K) -> np.ndarray:
     """Per-attempt latency (us) of a K-bubble system running alone on an SM
-    sub-partition; K > 8 extrapolated linearly in K."""
-    K = np.atleast_1d(np.asarray(K, dtype=np.float64))
-    ks = np.asarray(sorted(ALONE_US), dtype=np.float64)
-    vs = np.asarray([ALONE_US[int(k)] for k in ks])
-    out = np.interp(K, ks, vs)
-    big = K > ks[-1]
-    out[big] = vs[-1] * K[big] / ks[-1]
-    return out
+    sub-partition."""
+    return _per_bubble_count(ALONE_US, K)
 
 
 def make_work_list(K: np.ndarray, work: np.ndarray, active: Optional[np.ndarray] = None,
@@ -104,7 +101,7 @@ def make_work_list(K: np.ndarray, work: np.ndarray, active: Optional[np.ndarray]
 def with_latency_lane(wl: WorkList, K: np.ndarray, work: np.ndarray, fraction: float = 1e-3,
                       max_sms: int = 12) -> WorkList:
     """Moves the systems with the longest predicted serial time into latency
-    lanes: extra buckets of the same K whose blocks (4 warps) each hold an SM
+    lanes: extra buckets of the same K whose blocks each hold an SM
     alone, so their steps run at the minimum latency instead of sharing issue
     slots with a full SM.  The serial time of a system is its predicted steps
     times the per-step latency of its warp on a full GPU, which grows with the
@@ -115,7 +112,7 @@ def with_latency_lane(wl: WorkList, K: np.ndarray, work: np.ndarray, fraction: f
     if wl.order.size == 0 or max_sms < 1:
         return wl
     ids = wl.order
-    chain = work[ids] * cost_weight(K[ids]) * (32 // K[ids])
+    chain = work[ids] * alone_latency(K[ids])
     n_lat = int(np.ceil(fraction * ids.size))
     top = ids[np.argsort(-chain, kind="stable")[:n_lat]]
     # trim to the SM budget, keeping the longest chains
@@ -562,7 +559,7 @@ class AdaptivePlan:
       has not run enough steps to measure its own);
     * a system whose remaining attempts at the latency it sees outside a lane
       (its alone latency ``ALONE_US`` x ``load_factor``; the latency of one
-      attempt inside the full GPU is 1.31-1.48x the alone latency for
+      attempt inside the full GPU is 1.38-1.58x the alone latency for
       K = 3..8 on a full B200, ``bench.py --workload costs``, but 1.2 gave
       the shortest mixed-K solves of 1.0-1.35: every lane takes a whole SM
       from the bulk)
