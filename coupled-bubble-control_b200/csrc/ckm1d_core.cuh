@@ -1056,10 +1056,50 @@ __device__ __forceinline__ void candidate(const Params& P, bool on, double h, co
   ratio = r[2] < r[0] ? r[2] : r[0];
 }
 
+// State at Cash-Karp stage st.
+__device__ __forceinline__ void stage_state(int st, const double* ks, double h, const double y[4], double ys[4]) {
+  switch (st) {
+    case 0:
+#pragma unroll
+      for (int c = 0; c < 4; ++c) ys[c] = y[c];
+      break;
+    case 1: stage_state<1>(ks, h, y, ys); break;
+    case 2: stage_state<2>(ks, h, y, ys); break;
+    case 3: stage_state<3>(ks, h, y, ys); break;
+    case 4: stage_state<4>(ks, h, y, ys); break;
+    default: stage_state<5>(ks, h, y, ys); break;
+  }
+}
+
+// The six stages of an attempt with one field form of the right-hand side;
+// whether every state of this lane was within the range of the fast functions.
+template <int KB, int KC, int LIN, int NKC, int ACC, bool FAST>
+__device__ __forceinline__ bool six_stages(const Geo& g, const Params& P, const WarpSmem& W, const LaneState& S, bool on,
+                                           double h, int& sweeps, int& conv_fail) {
+  double* ks = W.ks + g.lane;
+  bool in_range = true;
+  conv_fail = sweeps = 0;
+#pragma unroll 1
+  for (int st = 0; st < 6; ++st) {
+    double ys[4], kk[4];
+    stage_state(st, ks, h, S.y, ys);
+    bool cv, ok;
+    int it;
+    rhs_form<KB, KC, LIN, NKC, ACC, FAST>(g, P, W, S.sp0, S.sp3, on, st == 0 ? S.t : fma(kStageA[st], h, S.t), ys, kk,
+                                          ok, cv, it);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) ks[(st * 4 + c) * 32] = kk[c];
+    in_range = in_range & ok;
+    sweeps += it;
+    conv_fail += cv ? 0 : 1;
+  }
+  return in_range;
+}
+
 // One adaptive Cash-Karp step for every active group of the warp
 // (stepper.py:362-677).  Returns true (per lane) if a dense sample must be
 // stored after this step; the caller writes it.
-template <int KB, int KC, int LIN>
+template <int KB, int KC, int LIN, bool HOISTED = false>
 __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSmem& W, LaneState& S) {
   const bool on = S.active;
   double h = S.h;
@@ -1087,9 +1127,13 @@ __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSm
   // branch never diverges), and so does a warp that holds a system outside the
   // range of the fast functions.  An attempt in which some state of the warp
   // left that range is evaluated again.
-  // The form is held in two flags, for two bubbles in one and P.ac (no register is
-  // left): an attempt alone in one flag / two, K = 2 10.2 us / 10.8 (16 bytes
-  // spilled), 3 13.4 / 12.6, 5 22.0 / 18.3, 6 22.9 / 18.4, 4, 7 and 8 the same.
+  // The choice is written in three ways, which differ in the code that the compiler
+  // makes of them: a loop over the stages per form (HOISTED), or one loop with the
+  // form in two flags (FLAGS) or in one and P.ac.  An attempt hoisted / one flag / two
+  // flags, two bubbles: reference layout alone 9.3 us / 10.3 / 10.0, 1,024 systems
+  // 11.0 / 12.0 / 11.6; batched with the GPU full 0.652 ns / 0.622 / 0.641 (16 bytes
+  // spilled).  Batched alone: 3 15.1 us / 13.4 / 12.6, 5 21.2 / 22.0 / 18.2,
+  // 6 22.7 / 22.9 / 18.5, 4, 7 and 8 the same.
   constexpr bool FAST = LIN == LIN_RICHARDSON, FLAGS = FAST && KB > 2;
   bool general = P.nk != 2 || P.ac == 0;
   if constexpr (FAST) {
@@ -1099,45 +1143,45 @@ __device__ __forceinline__ bool step(const Geo& g, const Params& P, const WarpSm
     const bool outside = __any_sync(FULL, on & !(reached <= fast_until_of(W, g, P.nk)));
     general = general | outside;
   }
-  bool swa = !general & (P.ac == 2), swn = !general & (P.ac == 1);
   int conv_fail_here, sweeps;
-  while (true) {
-    bool in_range = true;
-    conv_fail_here = sweeps = 0;
-#pragma unroll 1
-    for (int st = 0; st < 6; ++st) {
-      double ys[4];
-      switch (st) {
-        case 0:
-#pragma unroll
-          for (int c = 0; c < 4; ++c) ys[c] = S.y[c];
-          break;
-        case 1: stage_state<1>(ks, h, S.y, ys); break;
-        case 2: stage_state<2>(ks, h, S.y, ys); break;
-        case 3: stage_state<3>(ks, h, S.y, ys); break;
-        case 4: stage_state<4>(ks, h, S.y, ys); break;
-        default: stage_state<5>(ks, h, S.y, ys); break;
-      }
-      const double ts = (st == 0) ? t : fma(kStageA[st], h, t);
-      double kk[4];
-      bool cv, ok;
-      int it;
-      if (FLAGS ? swa : !general && P.ac == 2)
-        rhs_form<KB, KC, LIN, 2, 2, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
-      else if (FLAGS ? swn : !general)
-        rhs_form<KB, KC, LIN, 2, 1, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
-      else
-        rhs_form<KB, KC, LIN, 0, -1, false>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) ks[(st * 4 + c) * 32] = kk[c];
-      in_range = in_range & ok;
-      sweeps += it;
-      conv_fail_here += cv ? 0 : 1;
+  if constexpr (HOISTED) {
+    if (!general) {
+      bool in_range;
+      if (P.ac == 2) in_range = six_stages<KB, KC, LIN, 2, 2, FAST>(g, P, W, S, on, h, sweeps, conv_fail_here);
+      else in_range = six_stages<KB, KC, LIN, 2, 1, FAST>(g, P, W, S, on, h, sweeps, conv_fail_here);
+      if constexpr (FAST) general = !__all_sync(FULL, !on | in_range);
     }
-    if (!FAST || (FLAGS ? !(swa | swn) : general)) break;
-    if (__all_sync(FULL, !on | in_range)) break;
-    general = true;
-    swa = swn = false;
+    if (general) six_stages<KB, KC, LIN, 0, -1, false>(g, P, W, S, on, h, sweeps, conv_fail_here);
+  } else {
+    bool swa = !general & (P.ac == 2), swn = !general & (P.ac == 1);
+    while (true) {
+      bool in_range = true;
+      conv_fail_here = sweeps = 0;
+#pragma unroll 1
+      for (int st = 0; st < 6; ++st) {
+        double ys[4];
+        stage_state(st, ks, h, S.y, ys);
+        const double ts = (st == 0) ? t : fma(kStageA[st], h, t);
+        double kk[4];
+        bool cv, ok;
+        int it;
+        if (FLAGS ? swa : !general && P.ac == 2)
+          rhs_form<KB, KC, LIN, 2, 2, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
+        else if (FLAGS ? swn : !general)
+          rhs_form<KB, KC, LIN, 2, 1, FAST>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
+        else
+          rhs_form<KB, KC, LIN, 0, -1, false>(g, P, W, S.sp0, S.sp3, on, ts, ys, kk, ok, cv, it);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) ks[(st * 4 + c) * 32] = kk[c];
+        in_range = in_range & ok;
+        sweeps += it;
+        conv_fail_here += cv ? 0 : 1;
+      }
+      if (!FAST || (FLAGS ? !(swa | swn) : general)) break;
+      if (__all_sync(FULL, !on | in_range)) break;
+      general = true;
+      swa = swn = false;
+    }
   }
   if (on) {
     S.lin_iters += sweeps;

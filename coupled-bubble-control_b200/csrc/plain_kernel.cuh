@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(128, min_blocks_for(KB))
 
   for (long long it = 0; it < budget; ++it) {
     if (!__any_sync(FULL, S.active)) break;
-    const bool st = step<KB, KC, LIN>(g, P, W, S);
+    const bool st = step<KB, KC, LIN, KB == 2 && LIN == LIN_RICHARDSON>(g, P, W, S);
     if (st) ref_store_dense(L, S.t, S.y, g.li, s, S.idx);
     after_store(S, P, st);
   }
