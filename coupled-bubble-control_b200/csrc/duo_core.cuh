@@ -10,7 +10,7 @@
 // accumulation chains in registers (lane 0: partners d = 1, 2 mod 4, lane 1:
 // d = 3, 0 mod 4), so only the iterates move: 16 bytes a partner, and the two
 // half sums meet in one shuffle.  An attempt before and after: K = 32 alone 80 us, now
-// 48, GPU full 230 ns, now 119; K = 20 164 us and 396 ns, now 56 and 122.
+// 47, GPU full 230 ns, now 118; K = 20 164 us and 396 ns, now 57 and 123.
 //
 // Same operations in the same order as the one-lane form (ckm1d_core.cuh): the
 // chains and their tree, the ordered sums over the partners (lane 0 sums the two
@@ -90,7 +90,7 @@ struct DuoSmem {
   double* rr;    // [2][32]   squared residuals
   double* cm;    // [3][32][32] coupling coefficients of partner d = 1..32 (zero past K - 1)
   double* red;   // [2][4]    per-warp results of the step's reductions
-  int* claim;    // [2]       claimed system; whether the time slice is over
+  int* claim;    // [2]       for the batched worker
   LaneCold* own; // [64]
   Cold* cold;    // scalars of the system
 };

@@ -9,12 +9,13 @@
 //   * a work list orders the systems by K bucket, longest expected work first;
 //   * each warp holds floor(32/K) system slots; whenever a system finishes,
 //     its slot writes the result back and claims the next system of its bucket
-//     with one atomicAdd per warp, so lanes never idle while work remains;
-//   * one persistent kernel per K bucket (instantiated for KB = 2,4,8,16,32
-//     lanes per system slot), launched on forked streams so the buckets overlap
-//     and a bucket's tail is filled by the next bucket's warps.
+//     with one atomicAdd per warp, so lanes never idle while work remains (above
+//     16 bubbles with the Richardson solve a team of two warps holds one system);
+//   * one persistent kernel per K bucket, of the form for its bubble count,
+//     launched on forked streams so the buckets overlap and a bucket's tail is
+//     filled by the next bucket's warps.
 // Integration arithmetic is the same device code as the reference-layout
-// kernel (ckm1d_core.cuh), so results are bit-identical to the CPU oracle.
+// kernels, so results are bit-identical to the CPU oracle.
 #pragma once
 
 #include "cbc_internal.h"
@@ -485,6 +486,15 @@ __global__ void __launch_bounds__(DUO_THREADS * TEAMS, DUO_BLOCKS / TEAMS)
   extern __shared__ __align__(16) double smem[];
   const DuoGeo<TEAMS> g = make_duo_geo<TEAMS>(KC > 0 ? KC : K);
   const DuoSmem W = duo_smem(g, smem, P.nk);
+  // [0] claimed system, [1] whether the time slice is over.  A block of one team keeps
+  // them in static shared memory (run-time K spills 50 bytes then, 130 in dynamic
+  // memory: GPU full 122.2 ns an attempt against 123.5 for K = 20); a lane's block
+  // requests all that its SM has and may have none.
+  int* claim = W.claim;
+  if constexpr (TEAMS == 1) {
+    __shared__ int words[2];
+    claim = words;
+  }
   const long long deadline = budget_ns > 0 ? epoch[0] + budget_ns : 0;
   BubbleState S;
   S.c = W.cold;
@@ -498,10 +508,10 @@ __global__ void __launch_bounds__(DUO_THREADS * TEAMS, DUO_BLOCKS / TEAMS)
         const int n = begin + atomicAdd(head, 1);
         if (n < end) idx = order[n];
       }
-      W.claim[0] = idx;
+      claim[0] = idx;
     }
     duo_sync(g);
-    const int sys = W.claim[0];
+    const int sys = claim[0];
     if (sys < 0) break;
     const long long row = E.bubble_offset[sys] + (g.valid ? g.i : 0);
     if (g.tid == 0 && E.trace_load_ns) E.trace_load_ns[sys] = global_ns();
@@ -526,9 +536,9 @@ __global__ void __launch_bounds__(DUO_THREADS * TEAMS, DUO_BLOCKS / TEAMS)
     }
     while (S.active) {
       if (deadline != 0) {     // time slice over: stop after the current step
-        if (g.tid == 0) W.claim[1] = global_ns() >= deadline;
+        if (g.tid == 0) claim[1] = global_ns() >= deadline;
         duo_sync(g);
-        if (W.claim[1]) {
+        if (claim[1]) {
           S.status = ST_MAX_STEPS;
           S.active = false;
           break;
