@@ -446,7 +446,7 @@ def env_step_latency(dev_index: int, n_steps: int = 128, warmup: int = 3, envs_p
 
 
 def large_k_measure(dev_index: int, ns: int = 16384, periods: float = 0.5, peak_tflops: float = 0.0):
-    """Large-K dense output (K = 32, one warp per system, 64 samples per
+    """Large-K dense output (K = 32, two warps per system, 64 samples per
     period): one batched solve of `ns` systems over `periods` periods from
     resident inputs.  Reports system-periods/s, the FP64 roofline numerator
     and the HBM rate of the trajectory writes (dense samples + times)."""

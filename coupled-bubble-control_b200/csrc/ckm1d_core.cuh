@@ -75,8 +75,8 @@ static __constant__ double kStageB[6][5] = {{0, 0, 0, 0, 0},
 
 // Resident 128-thread blocks per SM the register allocation is tuned for, per
 // lanes-per-system instantiation (ptxas: KB=2 fits 128 registers and KB=4 168
-// without spills; KB=8 needs ~250; KB >= 16 keeps its pair arrays in local
-// memory either way).
+// without spills; KB=8 needs ~250; above, the direct solve alone, whose shared
+// memory admits one block).
 __host__ __device__ constexpr int min_blocks_for(int KB) { return KB <= 2 ? 4 : (KB <= 4 ? 3 : (KB <= 8 ? 2 : 1)); }
 
 // Register-budget variant MB of the batched kernels: MB = 1 asks ptxas for one
@@ -368,7 +368,6 @@ __host__ __device__ constexpr bool iterates_stored(int K) { return K == 8; }
 
 // Residual r = b - A v of the implicit coupling system for this lane's bubble,
 // A = I + off-diagonal partner blocks.  Partner distance d = 1..K-1 goes to
-// accumulation chain (d - 1) mod 4 (increasing d within a chain); the chains
 // accumulation chain (d - 1) mod 4 (increasing d within a chain); the chains
 // are then combined by the open pairwise tree.
 template <int KB, int KC>
@@ -678,7 +677,8 @@ __device__ __forceinline__ bool state_in_range(double x0, double x1, double D) {
 // a branch, as the special cases of the general functions do: the seven of a
 // K = 8 bubble's partners took 74 cycles each, one after the other.  A step attempt
 // before and after: K = 2 alone 13.6 us, now 11.1, K = 4 17.9, 15.5, K = 8 26.0,
-// 22.0; GPU full K = 2 0.650 ns, 0.630, K = 8 7.69, 7.23.
+// 22.0; GPU full K = 2 0.650 ns, 0.630, K = 8 7.69, 7.23 (with the branch-free ratios
+// and the stored iterates 10.4, 14.5, 20.4 us and 0.623, 6.62 ns).
 template <int KB, int KC, int LIN, int NKC, int ACC, bool FAST>
 __device__ __forceinline__ void rhs_form(const Geo& g, const Params& P, const WarpSmem& W,
                                          double sp0, double sp3, bool on, double t, const double y[4],

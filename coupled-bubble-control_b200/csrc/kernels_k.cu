@@ -2,9 +2,9 @@
 // instantiation: compiled once per (CBC_KB, CBC_KC) pair of dispatch_k, so that
 // the instantiations build in parallel.
 // Above 8 bubbles the matrix rows of a lane fill its registers, and tables that
-// the compiler may fold cost more of them (9 to 15 bubbles: 104 bytes spilled, 40
-// without; 16: 4, 0; direct solve: 254 registers, 194).  Up to 8 bubbles it is the
-// other way round (2 bubbles: 0 bytes folded, 24 without; direct solve 8, 242).
+// the compiler may fold cost more of them (9 to 15 bubbles: 88 bytes spilled, 64
+// without; 17 to 31: 54, 50; direct solve: 254 registers, 194).  Up to 8 bubbles it is
+// the other way round (2 bubbles: 0 bytes folded, 20 without; direct solve 0, 218).
 #if CBC_KB >= 16
 #define CBCM_TABLE_CONST
 #endif

@@ -3,9 +3,10 @@
 //
 // Without partners there is nothing to exchange: no shuffle, no shared record, no
 // reduction.  (The one-lane-per-bubble form spent them all the same: 9.7 us an
-// attempt alone, now 5.3; 60,000 systems 0.194 ns an attempt, now 0.167.  For two bubbles per lane the sweep itself gets faster,
-// 51 cycles against 75, but the tests' selects double per lane and the whole
-// attempt does not: 15.0 us with 32 systems a warp against 12.5 with 16.)  The
+// attempt alone, now 5.3; 300,000 systems 0.194 ns an attempt, now 0.162.  For two
+// bubbles per lane the sweep itself gets faster, 51 cycles against 75, but the tests'
+// selects double per lane and the whole attempt does not: 15.0 us with 32 systems a
+// warp against 12.5 with 16.)  The
 // iteration's solution is its right-hand side; the loop is kept because its
 // count and its outcome are results (a residual that is not a number never
 // converges).
@@ -18,7 +19,9 @@
 namespace cbc {
 
 constexpr int SOLO_THREADS = 128;  // largest block
-constexpr int SOLO_BLOCKS = 4;     // of it per SM: 128 registers a thread
+// Blocks per SM that the registers are limited for: 128 a thread.  Shared memory
+// admits four with one harmonic, three with two (15 KB a warp).
+constexpr int SOLO_BLOCKS = 4;
 
 // Shared memory of a warp, in doubles: every lane uses its own columns.
 struct SoloSmem {

@@ -8,7 +8,9 @@
 // room the scalars of a system, which an attempt touches once, live in shared
 // memory (cold_core.cuh).  K = 16 has a kernel of its own; any other K runs one
 // padded to 16 with zero coefficients and zero partners, without a branch per
-// partner (K = 11 alone: 99 us with the branches, now 62).
+// partner (K = 11 alone: 99 us with the branches, now 56 to 58).  Registers and
+// shared memory (24 KB a warp) admit two blocks of four warps per SM: two warps a
+// scheduler.
 #pragma once
 
 #include "cold_core.cuh"
